@@ -29,6 +29,7 @@ extern "C" {
 #define VBD_DEVERR_CONTACT_OVERFLOW 2   /* more contacts on one particle than contact slots */
 #define VBD_DEVERR_SINGULAR_SKIPPED 4   /* |det H| <= 1e-8: update skipped, as the reference does */
 #define VBD_DEVERR_BAD_CONTACT 8        /* a contact names a particle or shape out of range (ignored) */
+#define VBD_DEVERR_BARRIER 16           /* a wait between the CTAs of one sweep ran out: the step's results are void */
 
 /* Arithmetic of vbd_step. */
 #define VBD_PRECISION_FP32 0   /* FP32 throughout: the reference's arithmetic */

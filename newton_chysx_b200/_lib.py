@@ -25,6 +25,7 @@ VBD_NOALLOC_MAX_CONTACT_SLOTS = 4
 VBD_DEVERR_NONFINITE = 1
 VBD_DEVERR_CONTACT_OVERFLOW = 2
 VBD_DEVERR_SINGULAR_SKIPPED = 4
+VBD_DEVERR_BARRIER = 16
 VBD_DEVERR_BAD_CONTACT = 8
 
 PRECISION = {"fp32": 0, "mixed": 1, "fp64": 2}

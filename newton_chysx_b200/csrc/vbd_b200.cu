@@ -23,6 +23,7 @@
 #include "vbd_soft.h"
 #include "vbd_ell16_damped.h"
 #include "vbd_ell16_pair.h"
+#include "vbd_parts.h"
 #include "vbd_sc_persistent.h"
 #include "vbd_shapes.cuh"
 #include "vbd_warp.h"
@@ -223,6 +224,17 @@ struct VbdSolver {
   long long ell_faces = 0, ell_hinges = 0;
   bool ell_face_damping = false, ell_hinge_damping = false;
   std::vector<int> inst_start_of_vertex;  // first particle of each particle's instance
+  // split instances (vbd_parts.cu): parts_on replaces the kernels that schedule, layout and lanes name
+  bool parts_on = false;
+  PartsConfig parts;
+  PartsPlan plan;
+  bool parts_damped = false, parts_face_damped = false;
+  std::vector<int> color_of;
+  PartsView pt = {};
+  char* pt_blob = nullptr;
+  uint4 *pt_faceA = nullptr, *pt_faceB = nullptr, *pt_hinge = nullptr;
+  float* pt_kd = nullptr;
+  float4* pt_contact = nullptr;
   // adjoint work buffers (allocated by the first vbd_adjoint_step)
   void* adj_work = nullptr;
   size_t adj_work_bytes = 0;
@@ -246,7 +258,8 @@ struct VbdSolver {
                   range_ebase, face_nb, face_dm, face_mat, face_kd, hinge_idx, hinge_prop, hinge_kd, adj_work,
                   ell16_faceA, ell16_faceB, ell16_hinge, sc_pos_cd, sc_disp, sc_ts, ring_nslot, ring_base,
                   ring_vbase, ring_A, ring_B, ring_H, ring_hdr, ring_kd, spr_idx, spr_prop, spr_off, spr_adj, sspr_off,
-                  sspr_adj, spr_acc, tet_idx, tet_pose, tet_off, tet_adj, sc_estart, sc_world};
+                  sspr_adj, spr_acc, tet_idx, tet_pose, tet_off, tet_adj, sc_estart, sc_world, pt_blob, pt_faceA, pt_faceB, pt_hinge,
+                  pt_kd, pt_contact};
     for (void* p : ps)
       if (p) cudaFree(p);
     sc_release(sc);
@@ -636,6 +649,194 @@ RingView ring_view(const VbdSolver* h) {
   e.hdr = h->ring_hdr;
   e.kd = h->ring_kd;
   return e;
+}
+
+template <typename T>
+int upload(T** d, const std::vector<T>& h);
+
+// The records of the split-instance plan from the model's current materials, into the buffers that are there when
+// their sizes are the same (a captured graph keeps reading them).
+template <typename T>
+int upload_same(T** d, const std::vector<T>& h, bool have) {
+  if (!have || !*d) return upload_into(d, h);
+  return h.empty() || cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice) == cudaSuccess
+             ? VBD_OK
+             : VBD_ERR_CUDA;
+}
+
+int parts_input(VbdSolver* h, PartsInput& in, std::vector<float> buf[6]) {
+  const VbdModelDesc& m = h->md;
+  int rc;
+  if ((rc = download(buf[0], m.tri_poses_dev, size_t(4) * h->T)) ||
+      (rc = download(buf[1], m.tri_materials_dev, size_t(5) * h->T)) ||
+      (rc = download(buf[2], m.tri_areas_dev, size_t(h->T))) ||
+      (rc = download(buf[3], m.edge_rest_angle_dev, size_t(h->E))) ||
+      (rc = download(buf[4], m.edge_rest_length_dev, size_t(h->E))) ||
+      (rc = download(buf[5], m.edge_bending_properties_dev, size_t(2) * h->E)))
+    return rc;
+  in.V = h->V, in.T = h->T, in.E = h->E;
+  in.C = int(h->color_offsets.size()) - 1;
+  in.tri = h->h_tri.data(), in.edges = h->h_edges.data();
+  in.foff = h->h_foff.data(), in.fadj = h->h_fadj.data(), in.eoff = h->h_eoff.data(), in.eadj = h->h_eadj.data();
+  in.color_of = h->color_of.data();
+  in.pose = buf[0].data(), in.mat = buf[1].data(), in.area = buf[2].data();
+  in.rest_angle = buf[3].data(), in.rest_length = buf[4].data(), in.bending = buf[5].data();
+  return VBD_OK;
+}
+
+int upload_parts_records(VbdSolver* h, const PartsInput& in, bool have) {
+  bool damped = false, face_damped = false;
+  for (int e = 0; e < h->E; ++e) damped |= in.bending[2 * size_t(e)] > 0.f && in.bending[2 * size_t(e) + 1] > 0.f;
+  for (int t = 0; t < h->T; ++t) {
+    const float* m = in.mat + 5 * size_t(t);
+    face_damped |= (m[0] > 0.f || m[1] > 0.f) && m[2] > 0.f;
+  }
+  std::vector<uint4> fa, fb, hg;
+  std::vector<float> kd;
+  parts_records(in, h->plan, damped, fa, fb, hg, kd);
+  int rc;
+  if ((rc = upload_same(&h->pt_faceA, fa, have)) || (rc = upload_same(&h->pt_faceB, fb, have)) ||
+      (rc = upload_same(&h->pt_hinge, hg, have)) || (damped && (rc = upload_same(&h->pt_kd, kd, have))))
+    return rc;
+  h->parts_damped = damped;
+  h->parts_face_damped = face_damped;
+  return VBD_OK;
+}
+
+// The plan's arrays in one allocation and one copy.
+int upload_plan(VbdSolver* h) {
+  const PartsPlan& p = h->plan;
+  std::vector<char> blob;
+  std::vector<std::pair<const void**, size_t>> at;
+  const auto put = [&](const auto& v, const void** to) {
+    blob.resize((blob.size() + 15) / 16 * 16);
+    at.push_back({to, blob.size()});
+    const char* b = reinterpret_cast<const char*>(v.data());
+    blob.insert(blob.end(), b, b + v.size() * sizeof(v[0]));
+  };
+  PartsView& d = h->pt;
+  put(p.job_order, (const void**)&d.job_order), put(p.part_base, (const void**)&d.part_base);
+  put(p.vert, (const void**)&d.vert), put(p.start, (const void**)&d.start);
+  put(p.ghost_off, (const void**)&d.ghost_off), put(p.ghost, (const void**)&d.ghost);
+  put(p.ghost_part, (const void**)&d.ghost_part), put(p.nf, (const void**)&d.nf), put(p.ne, (const void**)&d.ne);
+  put(p.fbase, (const void**)&d.fbase), put(p.ebase, (const void**)&d.ebase);
+  const int rc = upload(&h->pt_blob, blob);
+  if (rc) return rc;
+  for (auto& a : at) *a.first = h->pt_blob + a.second;
+  return VBD_OK;
+}
+
+PartsView parts_view(const VbdSolver* h) {
+  PartsView p = h->pt;  // the plan's arrays
+  p.C = h->plan.C, p.P = h->plan.P, p.njobs = h->plan.njobs;
+  p.places = h->plan.most_places, p.most_own = h->plan.most_own;
+  p.faceA = h->pt_faceA, p.faceB = h->pt_faceB, p.hinge = h->pt_hinge;
+  p.hinge_kd = h->parts_damped ? h->pt_kd : nullptr;
+  p.face_damping = h->parts_face_damped;
+  p.contact = h->pt_contact;
+  p.queue = h->queue;
+  p.done = reinterpret_cast<unsigned*>(h->queue + kDoneStride);
+  return p;
+}
+
+const void* parts_kernel(const VbdSolver* h, bool damped) {
+  if (h->precision == VBD_PRECISION_FP64) return parts_fn<double, MODE_FP64>(h->parts.L, false, damped);
+  if (h->precision == VBD_PRECISION_MIXED) return parts_fn<float, MODE_MIXED>(h->parts.L, h->parts.wide, damped);
+  return parts_fn<float, MODE_FP32>(h->parts.L, h->parts.wide, damped);
+}
+
+// Decides whether instances are split (wstart: first particle of each world, then V) and builds the plan. Leaves
+// parts_on false where the one-CTA or per-color kernels stay the better ones or the plan does not exist.
+int build_parts(VbdSolver* h, const std::vector<int>& wstart) {
+  int dev = 0, sms = 0, optin = 0, cooperative = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  CK(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev));
+  const int V = h->V, C = int(h->color_offsets.size()) - 1, W = h->W;
+  if (C < 2 || C > kPartColors || h->prm.iterations < 1) return VBD_OK;
+  // Enough worlds keep three resident CTAs on every SM busy without a tail, and a world's records then stay with one
+  // CTA: with side U{16..128} one CTA per world takes 7.08, 10.1, 10.8 and 20.2 ms for 128, 512, 1,024 and 2,048
+  // worlds, the split 1.43, 5.3, 10.4 and 20.2 ms.
+  if (W >= 12 * sms) return VBD_OK;
+  const bool f64 = h->precision == VBD_PRECISION_FP64;
+  const size_t place = f64 ? sizeof(double4) : sizeof(float4);
+  const int narrow = f64 ? 384 : 512, most = f64 ? 384 : 896;  // threads of the two variants of k_parts
+  PartsConfig g;
+  // 64 particles per CTA at least; up to 16 CTAs form one cluster, whose barrier is the cheaper one (a 32 x 32 cloth:
+  // 148 us on one cluster of 16 against 163 us on 16 CTAs of a grid and 160 us on a cluster of 8)
+  g.P = std::min(sms, (V + 63) / 64);
+  g.grid = g.P > 16;
+  if (!g.grid) g.P = std::max(2, g.P);
+  if (g.grid && !cooperative) return VBD_OK;
+  // jobs of whole worlds, so that a color's run fills the threads of a CTA once (512 worlds: 5.3 ms with runs of 802,
+  // 5.7 ms with twice that, 6.4 and 7.2 ms with a half and a quarter)
+  const long long cap = (long long)most * g.P * C;
+  const int nj = int(std::max(1LL, std::min((long long)W, (V + cap - 1) / cap)));
+  if (!g.grid && nj > 1) return VBD_OK;
+  std::vector<int> job_v0 = {0};
+  for (int w = 1; w < W; ++w)
+    if ((long long)wstart[w] * nj >= (long long)V * (long long)job_v0.size()) job_v0.push_back(wstart[w]);
+  job_v0.push_back(V);
+  int per_color = 1;  // the longest run of a color in a part
+  {
+    std::vector<int> count(C);
+    for (size_t j = 0; j + 1 < job_v0.size(); ++j) {
+      std::fill(count.begin(), count.end(), 0);
+      for (int v = job_v0[j]; v < job_v0[j + 1]; ++v) ++count[h->color_of[v]];
+      for (int c = 0; c < C; ++c) per_color = std::max(per_color, (count[c] + g.P - 1) / g.P);
+    }
+  }
+  // as many lanes per vertex as leave one round of a run (256 x 256: 421 us with 4, 511 with 8 in two rounds, 469
+  // with 2); two lanes also where that takes the wide variant (512 x 512 mixed: 1.77 ms against 2.01 with 1)
+  g.L = 1;
+  while (g.L < 8 && per_color * g.L * 2 <= narrow) g.L *= 2;
+  if (!f64 && g.L == 1 && per_color * 2 <= most) g.L = 2;
+  g.block = std::min(most, std::max(64, (per_color * g.L + 31) / 32 * 32));
+  g.wide = !f64 && g.L <= 2 && g.block > narrow;
+  if (!g.wide) g.block = std::min(g.block, narrow);
+  std::vector<float> buf[6];
+  PartsInput in;
+  int rc = parts_input(h, in, buf);
+  if (rc) return rc;
+  if (!parts_plan(in, job_v0, g.P, g.L, h->plan)) return VBD_OK;
+  g.smem = place * size_t(h->plan.most_places) + (place + sizeof(int)) * size_t(h->plan.most_own);
+  if (g.smem + 2048 > size_t(optin)) return VBD_OK;
+  h->parts = g;
+  // a refresh may bring hinge damping: both variants have to fit
+  const void* fns[2] = {parts_kernel(h, false), parts_kernel(h, true)};
+  for (const void* fn : fns) {
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(g.smem)));
+    if (!g.grid && g.P > 8) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  }
+  int fit = 1 << 30;
+  for (const void* fn : fns) {
+    int n = 0;
+    if (g.grid) {
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, g.block, g.smem));
+      n = n * sms / g.P;
+    } else {
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = g.P;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(g.P);
+      cfg.blockDim = dim3(g.block);
+      cfg.dynamicSmemBytes = g.smem;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      CK(cudaOccupancyMaxActiveClusters(&n, fn, &cfg));
+    }
+    fit = std::min(fit, n);
+  }
+  if (fit < 1) return VBD_OK;
+  h->parts.blocks = g.P * (g.grid ? 1 : std::min(fit, h->plan.njobs));
+  if ((rc = upload_plan(h)) || (h->S > 0 && (rc = dalloc(&h->pt_contact, 3 * size_t(V)))) ||
+      (rc = upload_parts_records(h, in, false)))
+    return rc;
+  h->parts_on = true;
+  return VBD_OK;
 }
 
 Ell16View ell16_view(const VbdSolver* h) {
@@ -1193,6 +1394,13 @@ int step_impl(VbdSolver* h, R* q_in, R* q_out, const R* qd_in, R* qd_out, const 
       it = it1;
     } while (it < iters);
     CK(cudaGetLastError());
+  } else if (h->parts_on && !h->sc_on) {
+    CK(cudaMemsetAsync(h->queue, 0, sizeof(int) * (h->parts.grid ? size_t(kDoneStride) * (h->plan.P + 1) : 1), st));
+    if (has_c) {
+      CK(cudaMemsetAsync(h->slot_cnt, 0, sizeof(int) * h->V, st));
+      k_contact_prepare<R><<<(c.c_max + 255) / 256, 256, 0, st>>>(c);
+    }
+    CK((launch_parts<R, MODE>(h->parts, h->parts_damped, c, parts_view(h), iters, st)));
   } else if (h->schedule == VBD_SCHEDULE_PERSISTENT) {
     CK(cudaMemsetAsync(h->queue, 0, sizeof(int), st));
     if (has_c) {
@@ -1793,7 +2001,7 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
                    [&](int a, int b) { return wstart[a + 1] - wstart[a] > wstart[b + 1] - wstart[b]; });
   if ((rc = upload(&h->inst_order, order)) || (rc = upload(&h->inst_vstart, wstart)) ||
       (rc = upload(&h->inst_cptr, cptr)) || (rc = upload(&h->color_ranges, ranges)) ||
-      (rc = upload(&h->color_verts, verts)) || (rc = dalloc(&h->queue, 1)))
+      (rc = upload(&h->color_verts, verts)) || (rc = dalloc(&h->queue, size_t(kDoneStride) * 1025)))
     return fail(rc);
 
   // scratch
@@ -1875,7 +2083,20 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
     h->occ = params->min_blocks_per_sm;
     h->block = params->block_size ? params->block_size : 256;
   }
-  if (h->layout == VBD_LAYOUT_ELL || h->layout == VBD_LAYOUT_ELL16 || h->layout == VBD_LAYOUT_RING) {
+  // split instances: the default options, or the compact records on the persistent schedule. Options that name
+  // another kernel (the per-color schedule, another layout, lanes, a block size, shared positions off or on, pairs)
+  // keep it
+  const bool plain = params->layout == VBD_LAYOUT_AUTO && lpv == 0 && params->block_size == 0 &&
+                     params->min_blocks_per_sm == 0 && params->positions_in_shared == 0;
+  if (!soft && !lnh_floor && params->schedule != VBD_SCHEDULE_PER_COLOR && params->pair_vertices == 0 &&
+      params->instance_per_warp == 0 && (plain || h->layout == VBD_LAYOUT_ELL16)) {
+    h->color_of.assign(h->V, 0);
+    for (size_t col = 0; col + 1 < h->color_offsets.size(); ++col)
+      for (int k = h->color_offsets[col]; k < h->color_offsets[col + 1]; ++k) h->color_of[colp[k]] = int(col);
+    if ((rc = build_parts(h, wstart))) return fail(rc);
+  }
+  if (!h->parts_on &&
+      (h->layout == VBD_LAYOUT_ELL || h->layout == VBD_LAYOUT_ELL16 || h->layout == VBD_LAYOUT_RING)) {
     if (h->schedule == VBD_SCHEDULE_PERSISTENT) {
       h->range_verts_host = verts;
       h->ranges_host.clear();
@@ -1933,6 +2154,14 @@ int vbd_refresh_model(VbdHandle h, void* stream) {
     if ((rc = download(bp, h->md.edge_bending_properties_dev, size_t(2) * h->E))) return rc;
     for (int e = 0; e < h->E; ++e)
       if (bp[2 * e] > 0.f && bp[2 * e + 1] > 0.f) return VBD_ERR_UNSUPPORTED;
+  }
+  if (h->parts_on) {
+    if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) return VBD_ERR_CUDA;
+    std::vector<float> buf[6];
+    PartsInput in;
+    if ((rc = parts_input(h, in, buf))) return rc;
+    if (needs_lnh_floor(buf[1], h->T)) return VBD_ERR_UNSUPPORTED;
+    return upload_parts_records(h, in, true);
   }
   if (h->layout == VBD_LAYOUT_ELL || h->layout == VBD_LAYOUT_ELL16 || h->layout == VBD_LAYOUT_RING) {
     if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) return VBD_ERR_CUDA;
@@ -2020,7 +2249,7 @@ int vbd_get_residuals(VbdHandle h, double* out, int32_t n, void* stream) {
 int vbd_launches_per_step(VbdHandle h, int32_t* out) {
   if (!h || !out) return VBD_ERR_INVALID_ARGUMENT;
   const int C = int(h->color_offsets.size()) - 1, I = h->prm.iterations;
-  if (h->schedule == VBD_SCHEDULE_PERSISTENT) {
+  if (h->schedule == VBD_SCHEDULE_PERSISTENT || (h->parts_on && !h->sc_on)) {
     *out = 1 + (h->S > 0 ? 1 : 0);
   } else if (h->sc_on) {
     // kernels of this library per detection: 1 copy + per primitive kind (boxes, cell, count, fill, query)

@@ -291,14 +291,15 @@ __device__ __forceinline__ void contacts_add(const StepCtx<R>& c, int v, vec3<R>
 // the tangential part of the block is lost and the FP32 step of such a vertex can move it by metres. In FP64 the
 // stiff normal direction is a rank-one term known to 1e-16 and the tangential block survives. Vertices without
 // contacts solve in FP64 only when their FP32 block is ill-conditioned (|det H| < thr max|H|^3).
-template <typename R, int MODE>
-__device__ __forceinline__ double contacts_and_solve(const StepCtx<R>& c, int v, int ncont, vec3<R> x, vec3<R> f,
-                                                     sym3<R> H, const R* extra, vec3<R>& dlt, double& r2) {
-  if (MODE == MODE_MIXED && ncont > 0) {
+// add(x, f, H): adds the contact terms in the type of its arguments.
+template <typename R, int MODE, typename ADD>
+__device__ __forceinline__ double solve_with_contacts(const StepCtx<R>& c, bool contacts, const ADD& add, vec3<R> x,
+                                                      vec3<R> f, sym3<R> H, const R* extra, vec3<R>& dlt, double& r2) {
+  if (MODE == MODE_MIXED && contacts) {
     const vec3<double> xd = {double(x.x), double(x.y), double(x.z)};
     vec3<double> fd = {double(f.x), double(f.y), double(f.z)};
     sym3<double> Hd = {double(H.xx), double(H.yy), double(H.zz), double(H.xy), double(H.xz), double(H.yz)};
-    contacts_add_n<R, double>(c, v, ncont, xd, fd, Hd);
+    add(xd, fd, Hd);
     if (extra) {
       fd = fd + vec3<double>{double(extra[0]), double(extra[1]), double(extra[2])};
       Hd = Hd + sym3<double>{double(extra[3]), double(extra[4]), double(extra[5]),
@@ -310,7 +311,7 @@ __device__ __forceinline__ double contacts_and_solve(const StepCtx<R>& c, int v,
     dlt = {R(rr.x), R(rr.y), R(rr.z)};
     return det;
   }
-  if (ncont > 0) contacts_add_n<R>(c, v, ncont, x, f, H);
+  if (contacts) add(x, f, H);
   if (extra) {
     f = f + vec3<R>{extra[0], extra[1], extra[2]};
     H = H + sym3<R>{extra[3], extra[4], extra[5], extra[6], extra[7], extra[8]};
@@ -333,6 +334,13 @@ __device__ __forceinline__ double contacts_and_solve(const StepCtx<R>& c, int v,
   const R d = sdet(H);
   dlt = sadj_mul(H, f) * (R(1) / d);
   return double(d);
+}
+
+template <typename R, int MODE>
+__device__ __forceinline__ double contacts_and_solve(const StepCtx<R>& c, int v, int ncont, vec3<R> x, vec3<R> f,
+                                                     sym3<R> H, const R* extra, vec3<R>& dlt, double& r2) {
+  const auto add = [&](auto xa, auto& fa, auto& Ha) { contacts_add_n<R, decltype(xa.x)>(c, v, ncont, xa, fa, Ha); };
+  return solve_with_contacts<R, MODE>(c, ncont > 0, add, x, f, H, extra, dlt, r2);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -1,0 +1,87 @@
+// Split instances: the sweep of one cloth (or of a few, merged) by several CTAs at once, see vbd_parts.cu.
+#pragma once
+#include <vector>
+
+#include "vbd_ell.cuh"
+
+namespace vbd {
+
+// The device side of a plan. A job is a run of consecutive worlds; its particles are cut into P parts, one per CTA:
+// each color's particles, in index order, into P runs of equal length, so that every part has the same work in every
+// color (cuts by index alone give strips of a grid up to twice the average in some colors). A part keeps the positions of its own particles (by color, then by index) and of
+// the ghosts (other parts' particles that its elements touch, by color) in shared memory.
+struct PartsView {
+  int C;                      // colors
+  int P;                      // parts per job
+  int njobs;
+  int face_damping;           // some triangle is damped
+  int places, most_own;       // most places and most own particles of a part: the shared-memory layout
+  const int* job_order;       // [njobs] largest first
+  const int* part_base;       // [parts + 1] own particles of all parts before
+  const int* vert;            // [V] particle of part-local place s at part_base + s; bit 31: ghost of another part
+  const int* start;           // [parts, C + 1] own places by color
+  const int* ghost_off;       // [parts, C + 1] into ghost; a ghost's place is nown + (index - ghost_off[part, 0])
+  const int* ghost;           // particles
+  const int* ghost_part;      // the rank in the job of the part that owns each
+  const int* nf;              // [parts, C] face rounds of L lanes
+  const int* ne;              // [parts, C] hinge rounds
+  const long long* fbase;     // [parts, C] first face record
+  const long long* ebase;
+  const uint4* faceA;         // the records of vbd_ell.cuh's compact layout with part-local 16-bit places, round
+  const uint4* faceB;         //   major: base + (round * n + vertex) * L + lane
+  const uint4* hinge;
+  const float* hinge_kd;      // NULL without hinge damping
+  float4* contact;            // [3 V] by place: a particle's only contact with a static shape, as part_contact_add reads it
+  int* queue;                 // work counter, zero before launch
+  unsigned* done;             // [P * kDoneStride] colors finished by each CTA over its jobs, zero before launch (grid)
+};
+
+constexpr int kDoneStride = 32;  // one flag per 128-byte line
+
+constexpr int kPartColors = 32;  // most colors of a plan
+
+struct PartsConfig {
+  int P = 0;           // parts per job
+  bool grid = false;   // jobs in turn over the whole grid (cooperative launch); else a job per cluster
+  int L = 1;           // lanes per vertex
+  bool wide = false;   // the variant for up to 896 threads (72 registers) instead of 512 (128 registers)
+  int block = 0;
+  int blocks = 0;      // CTAs of the launch
+  size_t smem = 0;
+};
+
+template <typename R, int MODE>
+const void* parts_fn(int L, bool wide, bool damped);
+
+template <typename R, int MODE>
+cudaError_t launch_parts(const PartsConfig& g, bool damped, const StepCtx<R>& c, const PartsView& p, int iterations,
+                         cudaStream_t st);
+
+}  // namespace vbd
+
+namespace vbd {
+
+// The host side of a plan: the cut, the places, the ghosts and the record layout (topology only), and the records.
+struct PartsInput {
+  int V = 0, T = 0, E = 0, C = 0;
+  const int *tri = nullptr, *edges = nullptr;                                             // topology
+  const int *foff = nullptr, *fadj = nullptr, *eoff = nullptr, *eadj = nullptr;           // packed adjacency
+  const int* color_of = nullptr;                                                          // [V]
+  const float *pose = nullptr, *mat = nullptr, *area = nullptr;                           // triangles
+  const float *rest_angle = nullptr, *rest_length = nullptr, *bending = nullptr;          // hinges
+};
+struct PartsPlan {
+  int P = 0, L = 1, njobs = 0, C = 0, most_places = 0, most_own = 0;
+  std::vector<int> job_order, part_base, part_of, slot_of, vert, start, ghost_off, ghost, ghost_part, nf, ne;
+  std::vector<long long> fbase, ebase;
+  long long faces = 0, hinges = 0;
+};
+
+// Cuts the jobs (job_v0: first particle of each job, then V) into P parts each. False: the plan does not exist
+// (a part with 65,536 places or more, or an element that names a vertex twice, whose role the records cannot tell).
+bool parts_plan(const PartsInput& in, const std::vector<int>& job_v0, int P, int L, PartsPlan& plan);
+// The records of the plan's elements with the input's materials; kd stays empty when no hinge is damped.
+void parts_records(const PartsInput& in, const PartsPlan& plan, bool hinge_damping, std::vector<uint4>& faceA,
+                   std::vector<uint4>& faceB, std::vector<uint4>& hinge, std::vector<float>& kd);
+
+}  // namespace vbd

@@ -1,0 +1,155 @@
+"""Instances split over several CTAs (vbd_parts.cu) against the FP64 oracle and against the kernels they replace, at the
+edges of the rules that choose the split: one cluster and a grid, runs of one and two rounds, one to eight lanes per
+vertex, pinned ghosts, damping, several contacts per particle, worlds merged into jobs, refreshed materials, capture.
+
+Tolerances. FP64 sums in another order: 1e-9 m per substep, as the other FP64 kernels are held to. FP32 against FP64
+over one substep: 1e-4 m per m, the bound of every FP32 kernel here; on the finest sheets (2.4 mm cells under
+compression) the per-color FP32 kernel itself is 1.6e-4 m off, and the split one is held to twice that kernel's own
+distance, the factor for another order of the same sums."""
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+import newton_chysx_b200 as nb  # noqa: E402
+from newton_chysx_b200 import CollisionPipeline, SolverVBD  # noqa: E402
+from tests.helpers import cloth_grid_builder  # noqa: E402
+
+DT = 1.0 / 600.0
+
+
+def _sheet(nx, ny, kd=0.0, shapes=1):
+    b = nb.ModelBuilder(up_axis="Z", gravity=-9.81)
+    cell = 1.0 / max(nx - 1, ny - 1)
+    b.add_cloth_grid(pos=(0.0, 0.0, 4e-3), rot=nb.quat_identity(), vel=(0.0, 0.0, 0.0), dim_x=nx - 1, dim_y=ny - 1,
+                     cell_x=cell, cell_y=cell, mass=0.2 * cell * cell, tri_ke=4.0, tri_ka=3.0, tri_kd=kd,
+                     edge_ke=1e-4, edge_kd=kd, particle_radius=5e-3)  # fmt: skip
+    flags = b.particle_flags
+    flags[:: max(7, len(flags) // 9)] = 0  # pinned particles all over, so that some are ghosts
+    b.set_particle_flags(flags)
+    b.color(include_bending=True)
+    cfg = nb.ModelBuilder.ShapeConfig(ke=1e4, kd=1e-4, mu=0.5)
+    for k in range(shapes):
+        b.add_ground_plane(height=-1e-4 * k, cfg=cfg)
+    return b
+
+
+def _start(model, seed):
+    rng = np.random.default_rng(seed)
+    q = model.particle_q.cpu().numpy().astype(np.float64)
+    q = q * np.array([1.003, 1.002, 1.0]) + 2e-3 * np.sin(9.0 * q[:, [1, 0, 1]] + rng.uniform(0, 6, 3))
+    qd = np.array([0.2, -0.1, -0.4]) + 0.1 * np.sin(7.0 * q[:, [1, 0, 0]])
+    return q.astype(np.float32), qd.astype(np.float32)
+
+
+def _run(model, q, qd, substeps=2, **kw):
+    kw = dict(dict(iterations=6), **kw)
+    solver = SolverVBD(model, **kw)
+    f64 = kw.get("precision") == "fp64"
+    pipe = CollisionPipeline(model, soft_contact_margin=0.01)
+    contacts = pipe.contacts()
+    s0, s1, seen = model.state(), model.state(), model.state()
+    for s in (s0, s1):
+        if f64:
+            s.particle_f = None
+            s.particle_q, s.particle_qd = s.particle_q.double(), s.particle_qd.double()
+    s0.particle_q.copy_(torch.as_tensor(q))
+    s0.particle_qd.copy_(torch.as_tensor(qd))
+    for _ in range(substeps):
+        seen.particle_q.copy_(s0.particle_q)
+        pipe.collide(seen, contacts)
+        solver.step(s0, s1, None, contacts, DT)
+        s0, s1 = s1, s0
+    torch.cuda.synchronize()
+    assert solver.device_errors() == 0
+    return s0.particle_q.double().cpu().numpy(), s0.particle_qd.double().cpu().numpy()
+
+
+# 9 x 7: less than two CTAs' worth; 32 x 32: the largest cluster; 41 x 27: the first grid; 300 x 60: 148 CTAs with
+# eight lanes; 256 x 97 and 411 x 260: four and two lanes; 700 x 801: runs longer than a CTA's threads
+@pytest.mark.parametrize("nx,ny,kd,shapes", [(9, 7, 0.0, 1), (32, 32, 1e-3, 3), (41, 27, 0.0, 2), (300, 60, 1e-3, 1),
+                                              (256, 97, 0.0, 1), (411, 260, 0.0, 1), (700, 801, 0.0, 1)])  # fmt: skip
+def test_split_sheet_matches_the_per_color_kernels(nx, ny, kd, shapes):
+    model = _sheet(nx, ny, kd, shapes).finalize("cuda:0")
+    model.soft_contact_ke, model.soft_contact_kd, model.soft_contact_mu = 1e4, 1e-4, 0.5
+    q, qd = _start(model, nx)
+    ref, ref_d = _run(model, q, qd, precision="fp64", schedule="per_color")
+    got, got_d = _run(model, q, qd, precision="fp64")
+    assert np.abs(got - ref).max() <= 1e-9 and np.abs(got_d - ref_d).max() <= 1e-9 / DT
+    for precision in ("fp32", "mixed"):
+        got, _ = _run(model, q, qd, substeps=1, precision=precision)
+        old, _ = _run(model, q, qd, substeps=1, precision=precision, schedule="per_color")
+        one, _ = _run(model, q, qd, substeps=1, precision="fp64", schedule="per_color")
+        assert np.abs(got - one).max() <= max(1e-4, 2.0 * np.abs(old - one).max())
+
+
+@pytest.mark.parametrize("sides", [(5, 6), (17, 30, 8, 9, 21), (40,) * 30, (100, 128, 16, 90) * 6])
+def test_split_worlds_match_the_one_cta_kernel(sides):
+    top = nb.ModelBuilder(up_axis="Z", gravity=-9.81)
+    for n in sides:
+        top.add_world(_sheet(n, n, 1e-3 if n == 17 else 0.0, shapes=0))
+    top.add_ground_plane(cfg=nb.ModelBuilder.ShapeConfig(ke=1e4, kd=1e-4, mu=0.5))
+    model = top.finalize("cuda:0")
+    model.soft_contact_ke, model.soft_contact_kd, model.soft_contact_mu = 1e4, 1e-4, 0.5
+    q, qd = _start(model, len(sides))
+    ref, _ = _run(model, q, qd, precision="fp64", schedule="persistent", layout="ell")
+    got, _ = _run(model, q, qd, precision="fp64", schedule="persistent", layout="ell16")
+    assert np.abs(got - ref).max() <= 1e-9
+    got, _ = _run(model, q, qd, substeps=1, schedule="persistent", layout="ell16", min_blocks_per_sm=3)
+    ref, _ = _run(model, q, qd, substeps=1, precision="fp64", schedule="persistent", layout="ell")
+    assert np.abs(got - ref).max() <= 1e-4
+
+
+@pytest.mark.parametrize("n", [20, 64])
+def test_split_refresh_and_capture(n):
+    """A graph captured before a refresh steps with the new materials, hinge damping still off, and agrees with an
+    eager step bit for bit; a state stepped in place keeps working."""
+    model = _sheet(n, n).finalize("cuda:0")
+    q, qd = _start(model, n)
+    solver = SolverVBD(model, iterations=5)
+    pipe = CollisionPipeline(model, soft_contact_margin=0.01)
+    contacts = pipe.contacts()
+    s0, s1 = model.state(), model.state()
+
+    def reset():
+        s0.particle_q.copy_(torch.as_tensor(q))
+        s0.particle_qd.copy_(torch.as_tensor(qd))
+
+    reset()
+    pipe.collide(s0, contacts)
+    solver.step(s0, s1, None, contacts, DT)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream):
+        pipe.collide(s0, contacts)
+        solver.step(s0, s1, None, contacts, DT)
+    torch.cuda.synchronize()
+    model.tri_materials[:, :2] *= 3.0
+    solver.notify_model_changed()
+    reset()
+    graph.replay()
+    torch.cuda.synchronize()
+    captured = s1.particle_q.clone()
+    reset()
+    pipe.collide(s0, contacts)
+    solver.step(s0, s1, None, contacts, DT)
+    torch.cuda.synchronize()
+    assert torch.equal(captured, s1.particle_q)
+    fresh = SolverVBD(model, iterations=5)
+    reset()
+    pipe.collide(s0, contacts)
+    fresh.step(s0, s0, None, contacts, DT)
+    torch.cuda.synchronize()
+    assert torch.equal(captured, s0.particle_q)
+    del graph
+
+
+def test_split_leaves_explicit_shapes_and_small_models_alone():
+    b = cloth_grid_builder(n=12)
+    model = b.finalize("cuda:0")
+    assert SolverVBD(model, iterations=4, schedule="per_color").launches_per_step > 4
+    assert SolverVBD(model, iterations=4).launches_per_step <= 2
+    assert SolverVBD(model, iterations=0).launches_per_step <= 2
