@@ -15,7 +15,7 @@
 #include <vector>
 
 #include "vbd_b200.h"
-#include "vbd_adjoint.cuh"
+#include "vbd_adjoint.h"
 #include "vbd_contactgen.cuh"
 #include "vbd_collide.cuh"
 #include "vbd_ell.cuh"
@@ -229,7 +229,8 @@ struct VbdSolver {
   PartsConfig parts;
   PartsPlan plan;
   bool parts_damped = false, parts_face_damped = false;
-  std::vector<int> color_of;
+  std::vector<int> color_of;  // [V] place of each particle's color in the sweep
+  int* color_of_dev = nullptr;
   PartsView pt = {};
   char* pt_blob = nullptr;
   uint4 *pt_faceA = nullptr, *pt_faceB = nullptr, *pt_hinge = nullptr;
@@ -258,7 +259,7 @@ struct VbdSolver {
                   range_ebase, face_nb, face_dm, face_mat, face_kd, hinge_idx, hinge_prop, hinge_kd, adj_work,
                   ell16_faceA, ell16_faceB, ell16_hinge, sc_pos_cd, sc_disp, sc_ts, ring_nslot, ring_base,
                   ring_vbase, ring_A, ring_B, ring_H, ring_hdr, ring_kd, spr_idx, spr_prop, spr_off, spr_adj, sspr_off,
-                  sspr_adj, spr_acc, tet_idx, tet_pose, tet_off, tet_adj, sc_estart, sc_world, pt_blob, pt_faceA, pt_faceB, pt_hinge,
+                  sspr_adj, spr_acc, tet_idx, tet_pose, tet_off, tet_adj, sc_estart, sc_world, pt_blob, color_of_dev, pt_faceA, pt_faceB, pt_hinge,
                   pt_kd, pt_contact};
     for (void* p : ps)
       if (p) cudaFree(p);
@@ -1659,40 +1660,21 @@ int record_impl(VbdSolver* h, const R* q_in, const R* qd_in, const R* f_ext, con
   c.qd_out = qd_out;
   c.dt = dt;
   c.dt2r = R(1) / (dt * dt);
-  const int V = h->V, I = h->prm.iterations;
-  const size_t n3 = size_t(3) * V;
-  k_record_forward<R><<<(V + 255) / 256, 256, 0, st>>>(c, y);
-  if (has_c) {
-    CK(cudaMemsetAsync(h->slot_cnt, 0, sizeof(int) * V, st));
-    k_contact_prepare<R><<<(c.c_max + 255) / 256, 256, 0, st>>>(c);
-  }
-  CK(cudaMemcpyAsync(ck, y, n3 * sizeof(R), cudaMemcpyDeviceToDevice, st));
-  const int* cp = h->md.color_particles_dev;
-  for (int it = 0; it < I; ++it) {
-    R* cur = ck + size_t(it + 1) * n3;
-    CK(cudaMemcpyAsync(cur, ck + size_t(it) * n3, n3 * sizeof(R), cudaMemcpyDeviceToDevice, st));
-    for (size_t col = 0; col + 1 < h->color_offsets.size(); ++col) {
-      const int a = h->color_offsets[col], b = h->color_offsets[col + 1];
-      if (b > a) k_record_color<R><<<(b - a + 127) / 128, 128, 0, st>>>(c, cur, y, cur, cp + a, b - a);
-    }
-  }
-  k_record_finish<R><<<int((n3 + 255) / 256), 256, 0, st>>>(c, ck + size_t(I) * n3);
-  CK(cudaGetLastError());
+  CK((record_substep<R>(c, ColorLists{h->md.color_particles_dev, &h->color_offsets, h->color_of_dev},
+                        h->prm.iterations, y, ck, st)));
   return VBD_OK;
 }
 
 template <typename R>
 int adjoint_impl(VbdSolver* h, const R* q_in, const R* y, const R* ck, const VbdContactsDesc* contacts, R dt,
                  const R* aq_out, const R* aqd_out, R* aq_in, R* aqd_in, R* adj_mu, R* adj_lambda, cudaStream_t st) {
-  const int V = h->V, I = h->prm.iterations, C = int(h->color_offsets.size()) - 1;
-  const size_t n3 = size_t(3) * V;
   const bool has_c = contacts && contacts->soft_contact_max > 0 && contacts->soft_contact_count_dev;
   if (has_c) {
     if (h->prm.avbd_linear_beta != 0.f) return VBD_ERR_UNSUPPORTED;
     int rc = ensure_contact_capacity(h, contacts->soft_contact_max, st);
     if (rc) return rc;
   }
-  const size_t need = (size_t(std::max(C, 1)) + 3) * n3 * sizeof(R);
+  const size_t need = 3 * size_t(3) * h->V * sizeof(R);
   if (h->adj_work_bytes < need) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(st, &cs));
@@ -1704,41 +1686,14 @@ int adjoint_impl(VbdSolver* h, const R* q_in, const R* y, const R* ck, const Vbd
     if (rc) return rc;
     h->adj_work_bytes = need;
   }
-  R* S = (R*)h->adj_work;  // C color-start states
-  R* ax = S + size_t(std::max(C, 1)) * n3;
-  R* ay = ax + n3;
-  R* axp = ay + n3;
   StepCtx<R> c = make_ctx<R, MODE_FP32>(h);
   if (has_c) set_contacts(c, contacts);
   c.q_in = const_cast<R*>(q_in);
   c.dt = dt;
   c.dt2r = R(1) / (dt * dt);
-  k_adjoint_begin<R><<<int((n3 + 255) / 256), 256, 0, st>>>(int(n3), aq_out, aqd_out, R(1) / dt, ax, ay);
-  // this substep's start positions (damping and contact terms) and contact table, as its forward pass had them
-  k_adjoint_qprev<R><<<(V + 255) / 256, 256, 0, st>>>(c);
-  CK(cudaMemsetAsync(axp, 0, n3 * sizeof(R), st));
-  if (has_c) {
-    CK(cudaMemsetAsync(h->slot_cnt, 0, sizeof(int) * V, st));
-    k_contact_prepare<R><<<(c.c_max + 255) / 256, 256, 0, st>>>(c);
-  }
-  AdjCtx<R> A{c, nullptr, y, ax, ay, adj_mu, adj_lambda, axp};
-  const int* cp = h->md.color_particles_dev;
-  for (int it = I - 1; it >= 0; --it) {
-    CK(cudaMemcpyAsync(S, ck + size_t(it) * n3, n3 * sizeof(R), cudaMemcpyDeviceToDevice, st));
-    for (int col = 0; col + 1 < C; ++col) {
-      R* nxt = S + size_t(col + 1) * n3;
-      CK(cudaMemcpyAsync(nxt, S + size_t(col) * n3, n3 * sizeof(R), cudaMemcpyDeviceToDevice, st));
-      const int a = h->color_offsets[col], b = h->color_offsets[col + 1];
-      if (b > a) k_record_color<R><<<(b - a + 127) / 128, 128, 0, st>>>(c, nxt, y, nxt, cp + a, b - a);
-    }
-    for (int col = C - 1; col >= 0; --col) {
-      A.x = S + size_t(col) * n3;
-      const int a = h->color_offsets[col], b = h->color_offsets[col + 1];
-      if (b > a) k_adjoint_color<R><<<(b - a + 63) / 64, 64, 0, st>>>(A, cp + a, b - a);
-    }
-  }
-  k_adjoint_end<R><<<(V + 255) / 256, 256, 0, st>>>(c, ax, ay, axp, aqd_out, aq_in, aqd_in);
-  CK(cudaGetLastError());
+  CK((adjoint_substep<R>(c, ColorLists{h->md.color_particles_dev, &h->color_offsets, h->color_of_dev},
+                         h->prm.iterations, y, ck, (R*)h->adj_work, aq_out, aqd_out, aq_in, aqd_in, adj_mu, adj_lambda,
+                         st)));
   return VBD_OK;
 }
 
@@ -1933,10 +1888,12 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
   if ((rc = dalloc(&h->tri_idx, h->T)) || (rc = dalloc(&h->tri_pose, h->T)) || (rc = dalloc(&h->tri_mat, h->T)) ||
       (rc = dalloc(&h->edge_idx, h->E)) || (rc = dalloc(&h->edge_prop, h->E)))
     return fail(rc);
+  h->color_of.assign(h->V, 0);
+  for (size_t col = 0; col + 1 < h->color_offsets.size(); ++col)
+    for (int k = h->color_offsets[col]; k < h->color_offsets[col + 1]; ++k) h->color_of[colp[k]] = int(col);
+  if ((rc = upload(&h->color_of_dev, h->color_of))) return fail(rc);
   if (soft) {
-    std::vector<int> color_of(h->V, -1);
-    for (size_t col = 0; col + 1 < h->color_offsets.size(); ++col)
-      for (int k = h->color_offsets[col]; k < h->color_offsets[col + 1]; ++k) color_of[colp[k]] = int(col);
+    const std::vector<int>& color_of = h->color_of;
     std::vector<int> toff, tadj, soff, sadj, ssoff, ssadj;
     build_soft_adjacency(h->V, h->NT, tets.data(), h->NS, springs.data(), color_of, toff, tadj, soff, sadj, ssoff,
                          ssadj);
@@ -2090,9 +2047,6 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
                      params->min_blocks_per_sm == 0 && params->positions_in_shared == 0;
   if (!soft && !lnh_floor && params->schedule != VBD_SCHEDULE_PER_COLOR && params->pair_vertices == 0 &&
       params->instance_per_warp == 0 && (plain || h->layout == VBD_LAYOUT_ELL16)) {
-    h->color_of.assign(h->V, 0);
-    for (size_t col = 0; col + 1 < h->color_offsets.size(); ++col)
-      for (int k = h->color_offsets[col]; k < h->color_offsets[col + 1]; ++k) h->color_of[colp[k]] = int(col);
     if ((rc = build_parts(h, wstart))) return fail(rc);
   }
   if (!h->parts_on &&
