@@ -1231,7 +1231,7 @@ int sc_compact(ScBuffers& b, const int4* tri_idx, const int4* edge_idx, cudaStre
   CK(cudaMemsetAsync(b.ent_cnt, 0, sizeof(int) * (size_t(b.V) + 1), st));
   k_sc_entries<true><<<kScGridBlocks, 256, 0, st>>>(b.vt_off + b.V, b.ee_off + b.E, b.vt_pairs, b.ee_pairs,
                                                      b.ent_cnt, b.ent_off, b.ent, b.ecap, b.flags);
-  k_sc_sort_entries<<<(b.V + 127) / 128, 128, 0, st>>>(b.V, b.ent_off, b.ent);
+  k_sc_sort_entries<<<(b.V + kSortWarps - 1) / kSortWarps, 32 * kSortWarps, 0, st>>>(b.V, b.ent_off, b.ent);
   CK(cudaGetLastError());
   return VBD_OK;
 }
