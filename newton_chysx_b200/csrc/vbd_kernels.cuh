@@ -351,15 +351,13 @@ __device__ __forceinline__ void self_contact_add(const StepCtx<R>& c, const P& p
                                                  sym3<R>& H) {
   const int pair = int(code & 0x1FFFFFFFu), slot = int((code >> 29) & 3u);
   const int4 q = __ldg((code >> 31 ? c.ee_pairs : c.vt_pairs) + pair);
-  const int ids[4] = {q.x, q.y, q.z, q.w};
-  vec3<R> x[4], xa[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) x[k] = pos.ld(ids[k]), xa[k] = ld3<R>(c.qprev[ids[k]]);
+  const vec3<R> x[4] = {pos.ld(q.x), pos.ld(q.y), pos.ld(q.z), pos.ld(q.w)};
+  const auto start = [&](int k) { return ld3<R>(c.qprev[k == 0 ? q.x : (k == 1 ? q.y : (k == 2 ? q.z : q.w))]); };
   const R eps_u = c.fric_eps * c.dt;
   if (code >> 31)
-    sc_ee_add<R>(slot, x, xa, R(c.sc_radius), R(c.soft_ke), R(c.soft_kd), R(c.soft_mu), eps_u, c.dt, R(c.sc_ee_eps), f, H);
+    sc_ee_add<R>(slot, x, start, R(c.sc_radius), R(c.soft_ke), R(c.soft_kd), R(c.soft_mu), eps_u, c.dt, R(c.sc_ee_eps), f, H);
   else
-    sc_vt_add<R>(slot, x, xa, R(c.sc_radius), R(c.soft_ke), R(c.soft_kd), R(c.soft_mu), eps_u, c.dt, f, H);
+    sc_vt_add<R>(slot, x, start, R(c.sc_radius), R(c.soft_ke), R(c.soft_kd), R(c.soft_mu), eps_u, c.dt, f, H);
 }
 
 // Spring term of one entry (spring << 1) | end of vertex v's spring list.

@@ -175,16 +175,18 @@ __host__ __device__ __forceinline__ void sc_friction(R mu, R fn, vec3<R> n, vec3
   }
 }
 
-// Vertex-triangle pair, x = (a, b, c, p) current and xa at the start of the step. Adds the term of slot
-// `order` (0..2: triangle vertex, 3: the colliding vertex). Returns false when the pair is not in contact.
-template <typename R>
-__device__ __forceinline__ bool sc_vt_add(int order, const vec3<R> x[4], const vec3<R> xa[4], R radius, R ke, R kd, R mu,
+// Vertex-triangle pair, x = (a, b, c, p) current; start(k): the position of vertex k at the start of the step, read only
+// when the pair is in contact (most recorded pairs lie between the contact radius and the detection margin). Adds the
+// term of slot `order` (0..2: triangle vertex, 3: the colliding vertex). Returns false when the pair is not in contact.
+template <typename R, typename S>
+__device__ __forceinline__ bool sc_vt_add(int order, const vec3<R> x[4], const S& start, R radius, R ke, R kd, R mu,
                                           R eps_u, R dt, vec3<R>& f, sym3<R>& H) {
   R bary[3];
   const vec3<R> cp = tri_closest(x[0], x[1], x[2], x[3], bary);
   const vec3<R> diff = x[3] - cp;
   const R dis = length(diff);
   if (!(R(0) < dis && dis < radius)) return false;
+  const vec3<R> xa[4] = {start(0), start(1), start(2), start(3)};
   const vec3<R> n = diff * (R(1) / dis);
   R dEdD, d2E;
   sc_norm(dis, radius, ke, dEdD, d2E);
@@ -202,12 +204,13 @@ __device__ __forceinline__ bool sc_vt_add(int order, const vec3<R> x[4], const v
 }
 
 // Edge-edge pair, x = (e1.v0, e1.v1, e2.v0, e2.v1). Adds the term of e1's vertex `order` (0 or 1).
-template <typename R>
-__device__ __forceinline__ bool sc_ee_add(int order, const vec3<R> x[4], const vec3<R> xa[4], R radius, R ke, R kd, R mu,
+template <typename R, typename S>
+__device__ __forceinline__ bool sc_ee_add(int order, const vec3<R> x[4], const S& start, R radius, R ke, R kd, R mu,
                                           R eps_u, R dt, R ee_eps, vec3<R>& f, sym3<R>& H) {
   R s, t, dis;
   edge_closest(x[0], x[1], x[2], x[3], ee_eps, s, t, dis);
   if (!(R(0) < dis && dis < radius)) return false;
+  const vec3<R> xa[4] = {start(0), start(1), start(2), start(3)};
   const vec3<R> c1 = x[0] + (x[1] - x[0]) * s, c2 = x[2] + (x[3] - x[2]) * t;
   const vec3<R> n = (c1 - c2) * (R(1) / dis);
   R dEdD, d2E;
