@@ -82,6 +82,25 @@ __device__ __forceinline__ unsigned cell_hash(int x, int y, int z, int nb) {
   return ((unsigned)x * 73856093u ^ (unsigned)y * 19349663u ^ (unsigned)z * 83492791u) & unsigned(nb - 1);
 }
 
+// A primitive's lowest cell, kept in the w components of its box, and the cell coordinates of a key. A query meets a
+// primitive in up to eight cells and reports it from the one that holds the lower corner of the two boxes'
+// intersection; as a cell index grows with its coordinate, that cell is the larger of the two lowest cells per axis.
+__device__ __forceinline__ void keep_cell(float4* lo, float4* hi, long long key) {
+  lo->w = __int_as_float(int(key >> 32));
+  hi->w = __int_as_float(int(key));
+}
+__device__ __forceinline__ void keep_cell(double4* lo, double4*, long long key) { lo->w = __longlong_as_double(key); }
+__device__ __forceinline__ long long kept_cell(float4 lo, float4 hi) {
+  return ((long long)__float_as_int(lo.w) << 32) | (long long)unsigned(__float_as_int(hi.w));
+}
+__device__ __forceinline__ long long kept_cell(double4 lo, double4) { return __double_as_longlong(lo.w); }
+__device__ __forceinline__ int key_axis(long long key, int shift) {  // 21 bits, sign extended
+  return int((unsigned(key >> shift) & 0x1FFFFFu) << 11) >> 11;
+}
+__device__ __forceinline__ bool reports(long long kept, int x0, int y0, int z0, int cx, int cy, int cz) {
+  return max(x0, key_axis(kept, 42)) == cx && max(y0, key_axis(kept, 21)) == cy && max(z0, key_axis(kept, 0)) == cz;
+}
+
 // Primitive boxes (kind 0: triangles of tri_idx, kind 1: edges of edge_idx) and their size statistics.
 template <typename R>
 __global__ void k_sc_boxes(int kind, int P, const pos4_t<R>* __restrict__ pos, const int4* __restrict__ tri_idx,
@@ -130,7 +149,7 @@ static __global__ void k_sc_cell(double* stats, int P, double margin) {
 
 // insert (fill == false: count) every primitive into the cells its box overlaps
 template <typename R, bool FILL>
-__global__ void k_sc_grid(int P, const pos4_t<R>* __restrict__ lo, const pos4_t<R>* __restrict__ hi,
+__global__ void k_sc_grid(int P, pos4_t<R>* lo, pos4_t<R>* hi,
                           const double* __restrict__ stats, int nb, unsigned* bcount, const unsigned* __restrict__ bstart,
                           long long* ekey, int* eprim, long long gcap, int* flags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -138,6 +157,7 @@ __global__ void k_sc_grid(int P, const pos4_t<R>* __restrict__ lo, const pos4_t<
   const double inv = stats[3];
   const pos4_t<R> a = lo[i], b = hi[i];
   const int x0 = cell_of(double(a.x), inv), y0 = cell_of(double(a.y), inv), z0 = cell_of(double(a.z), inv);
+  if (!FILL) keep_cell(lo + i, hi + i, cell_key(x0, y0, z0));
   int x1 = cell_of(double(b.x), inv), y1 = cell_of(double(b.y), inv), z1 = cell_of(double(b.z), inv);
   if (x1 > x0 + 1 || y1 > y0 + 1 || z1 > z0 + 1) {  // not reachable with the cell size above
     atomicOr(flags + 3, 1);
@@ -274,16 +294,15 @@ __global__ void k_sc_query_vt(ScQuery s, const pos4_t<R>* __restrict__ pos, cons
           const int t = __ldg(s.eprim + e);
           const pos4_t<R> a = lo[t], b = hi[t];
           if (a.x > qhi.x || a.y > qhi.y || a.z > qhi.z || b.x < qlo.x || b.y < qlo.y || b.z < qlo.z) continue;
-          // report the pair from one cell only
-          if (cell_of(double(vmax(qlo.x, R(a.x))), inv) != cx || cell_of(double(vmax(qlo.y, R(a.y))), inv) != cy ||
-              cell_of(double(vmax(qlo.z, R(a.z))), inv) != cz)
-            continue;
+          if (!reports(kept_cell(a, b), x0, y0, z0, cx, cy, cz)) continue;  // report the pair from one cell only
           const int4 ti = __ldg(s.tri_idx + t);
           if (v == ti.x || v == ti.y || v == ti.z) continue;
           if (s.world && __ldg(s.world + ti.x) != __ldg(s.world + v)) continue;
-          if (sorted_contains(s.vt_foff, s.vt_f, v, t)) continue;
           R bary[3];
           const R dist = length(tri_closest(ld3<R>(pos[ti.x]), ld3<R>(pos[ti.y]), ld3<R>(pos[ti.z]), p, bary) - p);
+          // the distance before the filter: it needs no chain of dependent loads, and most boxes that overlap are
+          // further apart than the margin
+          if (!(dist < m) || sorted_contains(s.vt_foff, s.vt_f, v, t)) continue;
           if (s.rest_excl > 0.f) {
             const vec3<R> rv = rest_at<R>(s.rest_q, v);
             R rb[3];
@@ -291,12 +310,10 @@ __global__ void k_sc_query_vt(ScQuery s, const pos4_t<R>* __restrict__ pos, cons
                                               rest_at<R>(s.rest_q, ti.z), rv, rb) - rv);
             if (dref < R(s.rest_excl)) continue;
           }
-          if (dist < m) {
-            mn = vmin(mn, dist);
-            insert_smallest(list, min(cnt, s.vb), s.vb, t);
-            ++cnt;
-            if (s.tv) record_triangle_vertex(s, t, v, float(dist));
-          }
+          mn = vmin(mn, dist);
+          insert_smallest(list, min(cnt, s.vb), s.vb, t);
+          ++cnt;
+          if (s.tv) record_triangle_vertex(s, t, v, float(dist));
         }
       }
   if (cnt > s.vb) atomicOr(s.flags + 0, 1);
@@ -333,26 +350,22 @@ __global__ void k_sc_query_ee(ScQuery s, const pos4_t<R>* __restrict__ pos, cons
           const int f = __ldg(s.eprim + g);
           const pos4_t<R> a = lo[f], b = hi[f];
           if (a.x > qhi.x || a.y > qhi.y || a.z > qhi.z || b.x < qlo.x || b.y < qlo.y || b.z < qlo.z) continue;
-          if (cell_of(double(vmax(qlo.x, R(a.x))), inv) != cx || cell_of(double(vmax(qlo.y, R(a.y))), inv) != cy ||
-              cell_of(double(vmax(qlo.z, R(a.z))), inv) != cz)
-            continue;
+          if (!reports(kept_cell(a, b), x0, y0, z0, cx, cy, cz)) continue;
           const int4 fi = __ldg(s.edge_idx + f);
           if (ei.z == fi.z || ei.z == fi.w || ei.w == fi.z || ei.w == fi.w) continue;
           if (s.world && __ldg(s.world + fi.z) != __ldg(s.world + ei.z)) continue;
-          if (sorted_contains(s.ee_foff, s.ee_f, e, f)) continue;
           R ss, tt, dist;
           edge_closest(p0, p1, ld3<R>(pos[fi.z]), ld3<R>(pos[fi.w]), R(s.ee_eps), ss, tt, dist);
+          if (!(dist < m) || sorted_contains(s.ee_foff, s.ee_f, e, f)) continue;
           if (s.rest_excl > 0.f) {
             R rs, rt, dref;
             edge_closest(rest_at<R>(s.rest_q, ei.z), rest_at<R>(s.rest_q, ei.w), rest_at<R>(s.rest_q, fi.z),
                          rest_at<R>(s.rest_q, fi.w), R(s.ee_eps), rs, rt, dref);
             if (dref < R(s.rest_excl)) continue;
           }
-          if (dist < m) {
-            mn = vmin(mn, dist);
-            insert_smallest(list, min(cnt, s.eb), s.eb, f);
-            ++cnt;
-          }
+          mn = vmin(mn, dist);
+          insert_smallest(list, min(cnt, s.eb), s.eb, f);
+          ++cnt;
         }
       }
   if (cnt > s.eb) atomicOr(s.flags + 2, 1);
