@@ -178,6 +178,8 @@ struct VbdSolver {
   int NS = 0, NT = 0;
   bool soft = false;
   int n_same_springs = 0;
+  unsigned long long same_colors = 0;  // colors with springs inside them, see StepCtx
+  int* live = nullptr;
   int2* spr_idx = nullptr;
   float4* spr_prop = nullptr;
   int *spr_off = nullptr, *spr_adj = nullptr, *sspr_off = nullptr, *sspr_adj = nullptr;
@@ -259,7 +261,7 @@ struct VbdSolver {
                   range_ebase, face_nb, face_dm, face_mat, face_kd, hinge_idx, hinge_prop, hinge_kd, adj_work,
                   ell16_faceA, ell16_faceB, ell16_hinge, sc_pos_cd, sc_disp, sc_ts, ring_nslot, ring_base,
                   ring_vbase, ring_A, ring_B, ring_H, ring_hdr, ring_kd, spr_idx, spr_prop, spr_off, spr_adj, sspr_off,
-                  sspr_adj, spr_acc, tet_idx, tet_pose, tet_off, tet_adj, sc_estart, sc_world, pt_blob, color_of_dev, pt_faceA, pt_faceB, pt_hinge,
+                  sspr_adj, spr_acc, tet_idx, tet_pose, tet_off, tet_adj, sc_estart, sc_world, pt_blob, color_of_dev, live, pt_faceA, pt_faceB, pt_hinge,
                   pt_kd, pt_contact};
     for (void* p : ps)
       if (p) cudaFree(p);
@@ -869,6 +871,20 @@ EllView ell_view(const VbdSolver* h) {
   return e;
 }
 
+// Soft models: whether any triangle, any hinge has stiffness, for the kernels (StepCtx::live).
+int pack_live(VbdSolver* h) {
+  std::vector<float> tm, bp;
+  int rc;
+  if ((rc = download(tm, h->md.tri_materials_dev, size_t(5) * h->T)) ||
+      (rc = download(bp, h->md.edge_bending_properties_dev, size_t(2) * h->E)))
+    return rc;
+  int live[2] = {0, 0};
+  for (int t = 0; t < h->T; ++t) live[0] |= tm[5 * t] > 0.f || tm[5 * t + 1] > 0.f;
+  for (int e = 0; e < h->E; ++e) live[1] |= bp[2 * e] > 0.f;
+  CK(cudaMemcpy(h->live, live, sizeof(live), cudaMemcpyHostToDevice));
+  return VBD_OK;
+}
+
 int pack_model(VbdSolver* h, cudaStream_t st) {
   const VbdModelDesc& m = h->md;
   if (h->T > 0) {
@@ -1033,6 +1049,9 @@ StepCtx<R> make_ctx(VbdSolver* h) {
     c.sspr_off = h->sspr_off;
     c.sspr_adj = h->sspr_adj;
     c.n_same_springs = h->n_same_springs;
+    c.same_colors = h->same_colors;
+    c.color_of = h->color_of_dev;
+    c.live = h->live;
     c.spr_acc = (R*)h->spr_acc;
     c.tet_idx = h->tet_idx;
     c.tet_pose = h->tet_pose;
@@ -1320,6 +1339,10 @@ int ensure_contact_capacity(VbdSolver* h, int cmax, cudaStream_t st) {
   return VBD_OK;
 }
 
+bool same_color_springs(const VbdSolver* h, size_t color) {
+  return (h->same_colors >> std::min<size_t>(color, 63)) & 1ull;
+}
+
 template <typename R, int MODE>
 int step_impl(VbdSolver* h, R* q_in, R* q_out, const R* qd_in, R* qd_out, const R* f_ext,
               const VbdContactsDesc* contacts, const VbdBodyState* bodies, R dt, cudaStream_t st) {
@@ -1507,7 +1530,7 @@ int step_impl(VbdSolver* h, R* q_in, R* q_out, const R* qd_in, R* qd_out, const 
       for (size_t col = 0; col + 1 < h->color_offsets.size(); ++col) {
         const int a = h->color_offsets[col], b = h->color_offsets[col + 1];
         if (h->soft)
-          launch_color_soft<R, MODE>(true, h->L, c, cp + a, b - a, it, h->block, st);
+          launch_color_soft<R, MODE>(true, same_color_springs(h, col), h->L, c, cp + a, b - a, it, h->block, st);
         else
           launch_color_sc_any<R, MODE>(h->L, c, cp + a, b - a, it, h->block, st);
         sc_truncate<R>(h, st);
@@ -1525,7 +1548,7 @@ int step_impl(VbdSolver* h, R* q_in, R* q_out, const R* qd_in, R* qd_out, const 
         if (h->layout == VBD_LAYOUT_ELL) {
           if (b > a) k_color_ell<R, MODE><<<(b - a + h->block - 1) / h->block, h->block, 0, st>>>(c, e, cp + a, int(col), b - a, it);
         } else if (h->soft) {
-          launch_color_soft<R, MODE>(false, h->L, c, cp + a, b - a, it, h->block, st);
+          launch_color_soft<R, MODE>(false, same_color_springs(h, col), h->L, c, cp + a, b - a, it, h->block, st);
         } else {
           launch_color_any<R, MODE>(h->L, c, cp + a, b - a, it, h->block, st);
         }
@@ -1900,6 +1923,9 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
     build_soft_adjacency(h->V, h->NT, tets.data(), h->NS, springs.data(), color_of, toff, tadj, soff, sadj, ssoff,
                          ssadj);
     h->n_same_springs = ssoff[h->V];
+    for (int v = 0; v < h->V; ++v)
+      if (ssoff[v + 1] > ssoff[v]) h->same_colors |= 1ull << std::min(color_of[v], 63);
+    if ((rc = dalloc(&h->live, 2))) return fail(rc);
     const size_t racc = h->precision == VBD_PRECISION_FP64 ? sizeof(double) : sizeof(float);
     if ((rc = upload(&h->tet_off, toff)) || (rc = upload(&h->tet_adj, tadj)) || (rc = upload(&h->spr_off, soff)) ||
         (rc = upload(&h->spr_adj, sadj)) || (rc = upload(&h->sspr_off, ssoff)) || (rc = upload(&h->sspr_adj, ssadj)) ||
@@ -1908,7 +1934,7 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
       return fail(rc);
     if (h->n_same_springs && (rc = dalloc((char**)&h->spr_acc, racc * 9 * size_t(h->V)))) return fail(rc);
   }
-  if ((rc = pack_model(h, 0))) return fail(rc);
+  if ((rc = pack_model(h, 0)) || (soft && (rc = pack_live(h)))) return fail(rc);
 
   // instances (worlds)
   std::vector<int> wstart;
@@ -2105,6 +2131,10 @@ int vbd_refresh_model(VbdHandle h, void* stream) {
   if (!h) return VBD_ERR_INVALID_ARGUMENT;
   int rc = pack_model(h, (cudaStream_t)stream);
   if (rc) return rc;
+  if (h->soft) {
+    if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) return VBD_ERR_CUDA;
+    if ((rc = pack_live(h))) return rc;
+  }
   if (h->pair && h->E) {  // the paired kernel has no hinge damping term
     std::vector<float> bp;
     if ((rc = download(bp, h->md.edge_bending_properties_dev, size_t(2) * h->E))) return rc;
@@ -2205,6 +2235,8 @@ int vbd_get_residuals(VbdHandle h, double* out, int32_t n, void* stream) {
 int vbd_launches_per_step(VbdHandle h, int32_t* out) {
   if (!h || !out) return VBD_ERR_INVALID_ARGUMENT;
   const int C = int(h->color_offsets.size()) - 1, I = h->prm.iterations;
+  int pre = 0;  // spring pre-passes of an iteration
+  for (int c = 0; c < C; ++c) pre += same_color_springs(h, size_t(c));
   if (h->schedule == VBD_SCHEDULE_PERSISTENT || (h->parts_on && !h->sc_on)) {
     *out = 1 + (h->S > 0 ? 1 : 0);
   } else if (h->sc_on) {
@@ -2215,9 +2247,9 @@ int vbd_launches_per_step(VbdHandle h, int32_t* out) {
     for (int it = 0; it < I; ++it)
       if ((h->sc_interval == 0 && it == 0) || (h->sc_interval >= 1 && it % h->sc_interval == 0)) ++n_det;
     const bool duals = h->S > 0 && h->prm.avbd_linear_beta != 0.f;
-    *out = 2 + (h->S > 0 ? 1 : 0) + n_det * detect + 2 + I * (C * (h->n_same_springs ? 4 : 3) + (duals ? 1 : 0));
+    *out = 2 + (h->S > 0 ? 1 : 0) + n_det * detect + 2 + I * (C * 3 + pre + (duals ? 1 : 0));
   } else {
-    *out = 2 + (h->S > 0 ? 1 : 0) + I * C * (h->n_same_springs ? 2 : 1);
+    *out = 2 + (h->S > 0 ? 1 : 0) + I * (C + pre);
   }
   return VBD_OK;
 }

@@ -106,6 +106,9 @@ struct StepCtx {
   const int* __restrict__ sspr_off;     // [V+1] springs whose ends share a color (summed before the color's solve)
   const int* __restrict__ sspr_adj;
   int n_same_springs;                   // entries of sspr_adj; 0 = no pre-pass
+  unsigned long long same_colors;       // bit c: color c (63: any later one too) has such springs, the others need none
+  const int* __restrict__ color_of;     // [V]
+  const int* __restrict__ live;         // [2] whether any triangle, any hinge of the model has stiffness
   R* spr_acc;                           // [V, 9] pre-pass sums: f xyz, H xx yy zz xy xz yz
   const int4* __restrict__ tet_idx;
   const float4* __restrict__ tet_pose;  // [3 per tet]: rows of rest D^-1, w = mu, lambda, damping
@@ -424,8 +427,10 @@ __device__ __forceinline__ void solve_group(const StepCtx<R>& c, const P& pos, i
   if (active) {
     const int fb = __ldg(c.face_off + v), fe = __ldg(c.face_off + v + 1);
     const int eb = __ldg(c.edge_off + v), ee = __ldg(c.edge_off + v + 1);
-    const int nf = fe - fb;
-    int nfe = nf + (ee - eb);
+    // a soft body's surface triangles and hinges usually carry no stiffness: none of the model's does, none is visited
+    const int nf = SOFT && !__ldg(c.live) ? 0 : fe - fb;
+    const int nh = SOFT && !__ldg(c.live + 1) ? 0 : ee - eb;
+    int nfe = nf + nh;
     int tb = 0, nfet = nfe, sb = 0;
     if (SOFT) {
       tb = __ldg(c.tet_off + v);
@@ -461,7 +466,7 @@ __device__ __forceinline__ void solve_group(const StepCtx<R>& c, const P& pos, i
                           c.dt, xp, f, H);
         }
       }
-      for (int k = sub; k < ee - eb; k += L) {
+      for (int k = sub; k < nh; k += L) {
         const int a = __ldg(c.edge_adj + eb + k);
         const int e = a >> 2, ord = a & 3;
         const float4 pr = __ldg(c.edge_prop + e);
@@ -490,8 +495,8 @@ __device__ __forceinline__ void solve_group(const StepCtx<R>& c, const P& pos, i
         self_contact_add<R>(c, pos, __ldg(c.ent + cb + (it - nfe)), f, H);
       } else if (SOFT && it >= nfet) {
         spring_entry_add<R>(c, pos, v, __ldg(c.spr_adj + sb + (it - nfet)), f, H);
-      } else if (SOFT && it >= nf + (ee - eb)) {
-        tet_entry_add<R>(c, pos, __ldg(c.tet_adj + tb + (it - nf - (ee - eb))), f, H);
+      } else if (SOFT && it >= nf + nh) {
+        tet_entry_add<R>(c, pos, __ldg(c.tet_adj + tb + (it - nf - nh)), f, H);
       } else if (it < nf) {
         const int a = __ldg(c.face_adj + fb + it);
         const int t = a >> 2, ord = a & 3;
@@ -671,6 +676,13 @@ __global__ void k_contact_duals(StepCtx<R> c) {
   c.c_k[t] = float(vmin(R(c.c_k[t]) + c.beta * vmax(R(0), pen), R(c.c_ke[t])));
 }
 
+// Whether the color of the (non-empty) range [a, b) of verts has springs inside it.
+template <typename R>
+__device__ __forceinline__ bool needs_prepass(const StepCtx<R>& c, const int* __restrict__ verts, int a, int b) {
+  if (!c.same_colors || a >= b) return false;
+  return (c.same_colors >> min(__ldg(c.color_of + __ldg(verts + a)), 63)) & 1ull;
+}
+
 struct PersistentPlan {
   int W;                      // instances
   const int* inst_order;      // [W] processing order (largest first)
@@ -712,7 +724,7 @@ __global__ void k_persistent(StepCtx<R> c, PersistentPlan p) {
     for (int it = 0; it < p.iterations; ++it) {
       for (int col = cb; col + 1 < ce; ++col) {
         const int a = __ldg(p.color_ranges + col), b = __ldg(p.color_ranges + col + 1);
-        if (SOFT && c.n_same_springs) {
+        if (SOFT && needs_prepass(c, p.color_verts, a, b)) {
           for (int g = a + threadIdx.x; g < b; g += blockDim.x) spring_prepass_vertex<R>(c, pos, __ldg(p.color_verts + g));
           __syncthreads();
         }
@@ -760,7 +772,7 @@ __global__ void k_persistent_warp(StepCtx<R> c, PersistentPlan p, int slice) {
     for (int it = 0; it < p.iterations; ++it) {
       for (int col = cb; col + 1 < ce; ++col) {
         const int a = __ldg(p.color_ranges + col), b = __ldg(p.color_ranges + col + 1);
-        if (SOFT && c.n_same_springs) {
+        if (SOFT && needs_prepass(c, p.color_verts, a, b)) {
           for (int g = a + lane; g < b; g += 32) spring_prepass_vertex<R>(c, pos, __ldg(p.color_verts + g));
           __syncwarp();
         }

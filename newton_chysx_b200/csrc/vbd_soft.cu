@@ -27,9 +27,9 @@ static void launch_color_soft_sc(int L, const StepCtx<R>& c, const int* verts, i
 }
 
 template <typename R, int MODE>
-void launch_color_soft(bool sc, int L, const StepCtx<R>& c, const int* verts, int n, int it, int block,
+void launch_color_soft(bool sc, bool prepass, int L, const StepCtx<R>& c, const int* verts, int n, int it, int block,
                        cudaStream_t st) {
-  if (c.n_same_springs && n > 0) k_spring_prepass<R><<<(n + 127) / 128, 128, 0, st>>>(c, verts, n);
+  if (prepass && n > 0) k_spring_prepass<R><<<(n + 127) / 128, 128, 0, st>>>(c, verts, n);
   if (sc)
     launch_color_soft_sc<R, MODE, true>(L, c, verts, n, it, block, st);
   else
@@ -61,11 +61,11 @@ void launch_persistent_soft(int L, const StepCtx<R>& c, const PersistentPlan& p,
   }
 }
 
-template void launch_color_soft<float, MODE_FP32>(bool, int, const StepCtx<float>&, const int*, int, int, int,
+template void launch_color_soft<float, MODE_FP32>(bool, bool, int, const StepCtx<float>&, const int*, int, int, int,
                                                   cudaStream_t);
-template void launch_color_soft<float, MODE_MIXED>(bool, int, const StepCtx<float>&, const int*, int, int, int,
+template void launch_color_soft<float, MODE_MIXED>(bool, bool, int, const StepCtx<float>&, const int*, int, int, int,
                                                    cudaStream_t);
-template void launch_color_soft<double, MODE_FP64>(bool, int, const StepCtx<double>&, const int*, int, int, int,
+template void launch_color_soft<double, MODE_FP64>(bool, bool, int, const StepCtx<double>&, const int*, int, int, int,
                                                    cudaStream_t);
 template const void* persistent_soft_fn<float, MODE_FP32, true>(int);
 template const void* persistent_soft_fn<float, MODE_FP32, false>(int);

@@ -4,10 +4,10 @@
 
 namespace vbd {
 
-// One color of the per-color sweep: the same-color spring pre-pass (when the model has such springs) and
+// One color of the per-color sweep: the same-color spring pre-pass (when the color has such springs) and
 // the solve, with (sc = true) or without self-contact.
 template <typename R, int MODE>
-void launch_color_soft(bool sc, int L, const StepCtx<R>& c, const int* verts, int n, int it, int block,
+void launch_color_soft(bool sc, bool prepass, int L, const StepCtx<R>& c, const int* verts, int n, int it, int block,
                        cudaStream_t st);
 
 template <typename R, int MODE, bool SMEM>
