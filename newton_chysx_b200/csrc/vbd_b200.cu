@@ -177,6 +177,7 @@ struct VbdSolver {
   // springs and tetrahedra
   int NS = 0, NT = 0;
   bool soft = false;
+  bool soft_per_color = false;  // the automatic schedule chose per-color launches for a soft model (see vbd_create)
   int n_same_springs = 0;
   unsigned long long same_colors = 0;  // colors with springs inside them, see StepCtx
   int* live = nullptr;
@@ -759,9 +760,11 @@ int build_parts(VbdSolver* h, const std::vector<int>& wstart) {
   const int V = h->V, C = int(h->color_offsets.size()) - 1, W = h->W;
   if (C < 2 || C > kPartColors || h->prm.iterations < 1) return VBD_OK;
   // Enough worlds keep three resident CTAs on every SM busy without a tail, and a world's records then stay with one
-  // CTA: with side U{16..128} one CTA per world takes 7.08, 10.1, 10.8 and 20.2 ms for 128, 512, 1,024 and 2,048
-  // worlds, the split 1.43, 5.3, 10.4 and 20.2 ms.
-  if (W >= 12 * sms) return VBD_OK;
+  // CTA: with side U{16..128}, all particles in contact, one CTA per world takes 7.08, 10.1, 10.8 and 20.2 ms for 128,
+  // 512, 1,024 and 2,048 worlds, the split 1.43, 5.3, 10.4 and 20.2 ms. The line lies below the crossing, since
+  // solvers that step side by side on several streams fill each other's tails with one CTA per world and a split
+  // takes the whole GPU.
+  if (W >= 6 * sms) return VBD_OK;
   const bool f64 = h->precision == VBD_PRECISION_FP64;
   const size_t place = f64 ? sizeof(double4) : sizeof(float4);
   const int narrow = f64 ? 384 : 512, most = f64 ? 384 : 896;  // threads of the two variants of k_parts
@@ -2001,7 +2004,18 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
 
   // scheduling
   h->schedule = params->schedule;
-  if (h->schedule == VBD_SCHEDULE_AUTO) h->schedule = (h->W > 1 || h->V <= 4096) ? VBD_SCHEDULE_PERSISTENT : VBD_SCHEDULE_PER_COLOR;
+  if (h->schedule == VBD_SCHEDULE_AUTO) {
+    h->schedule = (h->W > 1 || h->V <= 4096) ? VBD_SCHEDULE_PERSISTENT : VBD_SCHEDULE_PER_COLOR;
+    // Soft bodies of more than 512 particles in few worlds: a color's tets keep many SMs busy, and one CTA per world takes
+    // a time that grows with the world. One block, default options, 10 iterations: 344 particles 367 us on one CTA and
+    // 397 per color, 1,332 particles 1,784 and 412, 4,097 particles 5,310 and 414; 16 worlds of 513: 632 and 597, 64:
+    // 657 and 762
+    int most = 0;
+    for (int w = 0; w < h->W; ++w) most = std::max(most, wstart[w + 1] - wstart[w]);
+    h->soft_per_color = soft && h->schedule == VBD_SCHEDULE_PERSISTENT && most > 512 && h->V <= 16384 && lpv == 0 &&
+                        params->block_size == 0 && params->positions_in_shared == 0 && params->instance_per_warp == 0;
+    if (h->soft_per_color) h->schedule = VBD_SCHEDULE_PER_COLOR;
+  }
   // default lanes per vertex: 8 for one persistent instance and for models with tetrahedra or springs (a
   // vertex of a tet mesh has ~11 incident tets; 8 lanes measured fastest on 4,096 blocks of 640 tets: 5.3 ms
   // per substep against 19.1 / 10.0 / 6.1 / 6.8 ms with 1 / 2 / 4 / 16), else 1 (one lane per stencil row)
@@ -2461,6 +2475,7 @@ int vbd_set_self_contact(VbdHandle h, const VbdSelfContactDesc* d) {
   if ((h->schedule != VBD_SCHEDULE_PER_COLOR && !persistent) || h->layout != VBD_LAYOUT_CSR) return VBD_ERR_UNSUPPORTED;
   // persistent: cloth only, the AVBD penalty fixed (its dual update would need a grid-wide pass per iteration)
   if (persistent && (h->soft || h->warp_inst || h->prm.avbd_linear_beta != 0.f)) return VBD_ERR_UNSUPPORTED;
+  if (h->soft_per_color) return VBD_ERR_UNSUPPORTED;  // as with the persistent schedule: ask for per_color
   const long long V = h->V, E = h->E;
   if (V * d->vertex_buffer_size >= (1LL << 29) || E * d->edge_buffer_size >= (1LL << 29) ||
       4 * V * d->vertex_buffer_size + 2 * E * d->edge_buffer_size >= (1LL << 31))

@@ -42,6 +42,33 @@ def _step(solver, model, q, qd):
     return b.particle_q.clone()
 
 
+@pytest.mark.parametrize("cells,worlds,schedule", [(6, 1, "persistent"), (8, 1, "per_color"), (8, 2, "per_color"),
+                                                    (8, 30, "persistent")])  # fmt: skip
+def test_automatic_schedule_of_soft_blocks(cells, worlds, schedule):
+    """344 particles in one world stay on one CTA, 730 take per-color launches up to 16,384 in all; options that the
+    per-color schedule does not take keep the persistent one. Either way the same step."""
+    one = nb.ModelBuilder(up_axis="Z", gravity=-9.81)
+    one.add_soft_grid(pos=(0.0, 0.0, 0.0), rot=nb.quat_identity(), vel=(0.0, 0.0, 0.0), dim_x=cells, dim_y=cells,
+                      dim_z=cells, cell_x=0.02, cell_y=0.02, cell_z=0.02, density=500.0, k_mu=2e4, k_lambda=3e4,
+                      k_damp=1e-3, particle_radius=2e-3)  # fmt: skip
+    one.color()
+    b = one
+    if worlds > 1:
+        b = nb.ModelBuilder(up_axis="Z", gravity=-9.81)
+        for _ in range(worlds):
+            b.add_world(one)
+    model = b.finalize("cuda:0")
+    rng = np.random.default_rng(cells)
+    q = model.particle_q.double() + torch.as_tensor(1e-3 * rng.normal(size=(model.particle_count, 3)), device="cuda:0")
+    qd = torch.zeros_like(q)
+    solver = SolverVBD(model, iterations=3, precision="fp64")
+    assert solver.schedule == schedule
+    assert SolverVBD(model, iterations=3, block_size=256).schedule == "persistent"
+    other = "per_color" if schedule == "persistent" else "persistent"
+    ref = _step(SolverVBD(model, iterations=3, precision="fp64", schedule=other), model, q, qd)
+    assert float((_step(solver, model, q, qd) - ref).abs().max()) <= 1e-9
+
+
 @pytest.mark.parametrize("schedule", ["per_color", "persistent"])
 @pytest.mark.parametrize("same_color_spring", [False, True])
 def test_surface_stiffness_comes_and_goes(schedule, same_color_spring):
