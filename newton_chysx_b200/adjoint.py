@@ -1,8 +1,9 @@
 """Differentiable VBD substeps: the hand-written adjoint of the C ABI behind ``torch.autograd``.
 
 ``vbd_step`` has a hand-written reverse, ``vbd_adjoint_step``. Its forward pass ``vbd_record_step``
-keeps the positions at the start of every iteration (per-iteration checkpoints). The reverse pass
-recomputes the per-color states of one iteration from its checkpoint and walks the colors backwards.
+keeps the positions at the start of every iteration (per-iteration checkpoints). The reverse pass walks the
+colors backwards; a color's start state is read from two consecutive checkpoints, since within an iteration a
+vertex moves once, in its own color.
 Gradients flow to the input positions and velocities and to the triangles' Lame coefficients
 (``Model.tri_materials[:, 0:2]``), hence to anything they are computed from, e.g. per-triangle
 Young's moduli. Membranes, hinges, tetrahedra and springs take part with their damping.

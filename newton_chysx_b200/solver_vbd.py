@@ -24,6 +24,8 @@ Beyond the reference keywords:
   256 threads per SM (a register budget); 0 leaves the compiler's choice.
 * ``pair_vertices``: the ell16 persistent kernel (FP32) solves two vertices per thread, one in each lane
   of Blackwell's paired FP32 instructions (FFMA2 / FADD2 / FMUL2), halving the arithmetic instructions.
+* Cloths with default options, and ell16 batches of fewer than six worlds per SM, run split over several CTAs each
+  (one launch per substep); ``schedule``, ``layout`` and ``lanes_per_vertex`` then name what they would take unsplit.
 * ``instance_per_warp``: the persistent csr kernel gives each warp its own instance (colors separated by
   ``__syncwarp`` instead of a CTA barrier), for batches of small instances such as soft-body blocks.
 
