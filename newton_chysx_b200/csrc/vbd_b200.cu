@@ -143,7 +143,7 @@ static_assert(kMaxContactShapes == kParamTableShapes, "one parameter-table size"
 namespace {
 void sc_release(ScBuffers& b) {
   void* ps[] = {b.bcount, b.bstart, b.ekey, b.eprim, b.blo, b.bhi, b.stats, b.vt_tri, b.vt_count, b.vt_min,
-                b.ee_edge, b.ee_count, b.ee_min, b.flags, b.tmp, b.vt_off, b.vt_pairs, b.ee_off, b.ee_once, b.ee_pairs,
+                b.ee_edge, b.ee_count, b.ee_min, b.flags, b.tmp, b.vt_off, b.vt_pairs, b.ee_off, b.ee_pairs,
                 b.ent_cnt, b.ent_off, b.ent, b.vt_foff, b.vt_f, b.ee_foff, b.ee_f, b.scan_tmp};
   for (void* p : ps)
     if (p) cudaFree(p);
@@ -1168,7 +1168,7 @@ int sc_alloc(ScBuffers& b, int V, int T, int E, int vb, int eb) {
       (rc = dalloc(&b.ee_count, size_t(E))) || (rc = dalloc((R**)&b.ee_min, size_t(E))) ||
       (rc = dalloc(&b.flags, 4)) || (rc = dalloc(&b.tmp, size_t(std::max(V, E)) + 1)) ||
       (rc = dalloc(&b.vt_off, size_t(V) + 1)) || (rc = dalloc(&b.vt_pairs, size_t(V) * vb)) ||
-      (rc = dalloc(&b.ee_off, size_t(E) + 1)) || (rc = dalloc(&b.ee_once, size_t(E) + 1)) || (rc = dalloc(&b.ee_pairs, size_t(E) * eb)) ||
+      (rc = dalloc(&b.ee_off, size_t(E) + 1)) || (rc = dalloc(&b.ee_pairs, size_t(E) * eb)) ||
       (rc = dalloc(&b.ent_cnt, size_t(V) + 1)) || (rc = dalloc(&b.ent_off, size_t(V) + 1)) ||
       (rc = dalloc(&b.ent, size_t(b.ecap))))
     return rc;
@@ -1239,14 +1239,12 @@ int sc_compact(ScBuffers& b, const int4* tri_idx, const int4* edge_idx, cudaStre
   k_sc_stored<<<(b.V + 256) / 256, 256, 0, st>>>(b.V, b.vb, b.vt_count, b.tmp);
   if ((rc = scan<int>(b, b.tmp, b.vt_off, b.V + 1, st))) return rc;
   if (b.V)
-    k_sc_pairs<false><<<(b.V + 255) / 256, 256, 0, st>>>(b.V, b.vb, b.vt_count, b.vt_tri, b.vt_off, nullptr, tri_idx, edge_idx,
+    k_sc_pairs<false><<<(b.V + 255) / 256, 256, 0, st>>>(b.V, b.vb, b.vt_count, b.vt_tri, b.vt_off, tri_idx, edge_idx,
                                                           b.vt_pairs);
   k_sc_stored<<<(b.E + 256) / 256, 256, 0, st>>>(b.E, b.eb, b.ee_count, b.tmp);
   if ((rc = scan<int>(b, b.tmp, b.ee_off, b.E + 1, st))) return rc;
-  k_sc_once<<<(b.E + 128) / 128, 128, 0, st>>>(b.E, b.eb, b.ee_count, b.ee_edge, b.tmp);
-  if ((rc = scan<int>(b, b.tmp, b.ee_once, b.E + 1, st))) return rc;
   if (b.E)
-    k_sc_pairs<true><<<(b.E + 255) / 256, 256, 0, st>>>(b.E, b.eb, b.ee_count, b.ee_edge, b.ee_off, b.ee_once, tri_idx, edge_idx,
+    k_sc_pairs<true><<<(b.E + 255) / 256, 256, 0, st>>>(b.E, b.eb, b.ee_count, b.ee_edge, b.ee_off, tri_idx, edge_idx,
                                                          b.ee_pairs);
   CK(cudaMemsetAsync(b.ent_cnt, 0, sizeof(int) * (size_t(b.V) + 1), st));
   k_sc_entries<false><<<kScGridBlocks, 256, 0, st>>>(b.vt_off + b.V, b.ee_off + b.E, b.vt_pairs, b.ee_pairs,
@@ -1299,7 +1297,7 @@ int sc_collide(VbdSolver* h, const R* q_state, cudaStream_t st) {
 template <typename R>
 void sc_truncate(VbdSolver* h, cudaStream_t st) {
   ScBuffers& b = h->sc;
-  k_sc_trunc_pairs<R><<<kScGridBlocks, 256, 0, st>>>(b.vt_off + b.V, b.ee_once + b.E, b.vt_pairs, b.ee_pairs,
+  k_sc_trunc_pairs<R><<<kScGridBlocks, 256, 0, st>>>(b.vt_off + b.V, b.ee_off + b.E, b.vt_pairs, b.ee_pairs,
                                                       (const pos4_t<R>*)h->sc_pos_cd,
                                                       (const pos4_t<R>*)h->sc_disp, R(h->sc_ee_eps), R(h->sc_relax),
                                                       (R*)h->sc_ts);
@@ -1407,7 +1405,7 @@ int step_impl(VbdSolver* h, R* q_in, R* q_out, const R* qd_in, R* qd_out, const 
     }
     PersistentPlan p{h->W, h->inst_order, h->inst_vstart, h->inst_cptr, h->color_ranges, h->color_verts, h->queue,
                      iters};
-    ScPersistentPlan s{h->sc_estart, h->sc.vt_off, h->sc.ee_once, h->sc.vt_pairs, h->sc.ee_pairs, h->sc_ts,
+    ScPersistentPlan s{h->sc_estart, h->sc.vt_off, h->sc.ee_off, h->sc.vt_pairs, h->sc.ee_pairs, h->sc_ts,
                        h->sc_ee_eps, h->sc_relax, h->sc_margin * h->sc_relax * 0.5, 0, 0, 0, 0};
     CK(cudaMemsetAsync(h->queue, 0, sizeof(int), st));
     launch_persistent_sc<R, MODE>(h->L, c, p, s, h->grid_sc, h->block, st);
@@ -2255,8 +2253,8 @@ int vbd_launches_per_step(VbdHandle h, int32_t* out) {
     *out = 1 + (h->S > 0 ? 1 : 0);
   } else if (h->sc_on) {
     // kernels of this library per detection: 1 copy + per primitive kind (boxes, cell, count, fill, query)
-    // + compaction (2 x (stored, pairs), mirrors + entry count, fill, sort); the seven cub scans are not counted
-    const int detect = 1 + 2 * 5 + 5 + 3;
+    // + compaction (2 x (stored, pairs) + entry count, fill, sort); the six cub scans are not counted
+    const int detect = 1 + 2 * 5 + 4 + 3;
     int n_det = 1;
     for (int it = 0; it < I; ++it)
       if ((h->sc_interval == 0 && it == 0) || (h->sc_interval >= 1 && it % h->sc_interval == 0)) ++n_det;

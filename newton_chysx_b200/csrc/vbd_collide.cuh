@@ -55,7 +55,6 @@ struct ScBuffers {
   int* vt_off = nullptr;         // [V + 1]
   int4* vt_pairs = nullptr;      // [V * vb] the pair's vertices: the triangle's three, then the vertex
   int* ee_off = nullptr;         // [E + 1]
-  int* ee_once = nullptr;        // [E + 1] of them, pairs before edge e that stand once or first (see sc_mirrored)
   int4* ee_pairs = nullptr;      // [E * eb] the pair's vertices: the edge's two, then the other edge's two
   int* ent_cnt = nullptr;        // [V + 1] entries per vertex, then fill cursors
   int* ent_off = nullptr;        // [V + 1]
@@ -380,55 +379,22 @@ static __global__ void k_sc_stored(int P, int cap, const int* __restrict__ count
   if (i == P) tmp[i] = 0;
 }
 
-// Two edges in contact find each other, so most edge-edge pairs stand twice, as (e, f) and (f, e). The solve needs both,
-// each for its first edge's vertices. The truncation needs one: the division plane of (f, e) is that of (e, f) with the
-// normal and the two sides exchanged, and the step fractions of the four vertices are the same. (e, f) with f < e is the
-// mirror of a pair when f's list holds e (a full list may have lost it).
-__device__ __forceinline__ bool sc_mirrored(int e, int f, int cap, const int* __restrict__ count,
-                                            const int* __restrict__ list) {
-  if (f >= e) return false;
-  const int* l = list + size_t(f) * cap;
-  int lo = 0, hi = min(__ldg(count + f), cap);
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (__ldg(l + mid) < e)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return lo < min(__ldg(count + f), cap) && __ldg(l + lo) == e;
-}
-
-// tmp[e] = stored pairs of edge e that are no mirrors (tmp[E] = 0 for the scan)
-static __global__ void k_sc_once(int E, int cap, const int* __restrict__ count, const int* __restrict__ list, int* tmp) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e > E) return;
-  int once = 0;
-  if (e < E) {
-    const int n = min(count[e], cap);
-    for (int k = 0; k < n; ++k) once += !sc_mirrored(e, list[size_t(e) * cap + k], cap, count, list);
-  }
-  tmp[e] = once;
-}
-
 // Dense pair lists: each pair stored as its four vertex ids, so that the solve and the truncation read a pair's
 // positions one load after its entry. VT (vertex i, triangle t): (t0, t1, t2, i); EE (edge i, edge j): the
-// vertices of i, then those of j. EE pairs that are no mirrors come first, by edge, then the mirrors (once: pairs before
-// each edge that are none), so that the truncation runs over the head of the list.
+// vertices of i, then those of j.
 template <bool EE>
 __global__ void k_sc_pairs(int P, int cap, const int* __restrict__ count, const int* __restrict__ list,
-                           const int* __restrict__ off, const int* __restrict__ once,
-                           const int4* __restrict__ tri_idx, const int4* __restrict__ edge_idx, int4* pairs) {
+                           const int* __restrict__ off, const int4* __restrict__ tri_idx,
+                           const int4* __restrict__ edge_idx, int4* pairs) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P) return;
   const int n = min(count[i], cap), o = off[i];
-  int head = EE ? once[i] : 0, tail = EE ? once[P] + o - head : 0;
   const int4 a = EE ? __ldg(edge_idx + i) : make_int4(0, 0, 0, 0);
   for (int k = 0; k < n; ++k) {
     const int j = list[size_t(i) * cap + k];
     if (EE) {
       const int4 b = __ldg(edge_idx + j);
-      pairs[sc_mirrored(i, j, cap, count, list) ? tail++ : head++] = make_int4(a.z, a.w, b.z, b.w);
+      pairs[o + k] = make_int4(a.z, a.w, b.z, b.w);
     } else {
       const int4 t = __ldg(tri_idx + j);
       pairs[o + k] = make_int4(t.x, t.y, t.z, i);

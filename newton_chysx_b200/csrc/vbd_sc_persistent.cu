@@ -16,7 +16,7 @@ template <typename R>
 __device__ __forceinline__ void truncate_instance(const StepCtx<R>& c, const ScPersistentPlan& s, int vs, int ve,
                                                   int es, int ee) {
   const int p0 = __ldg(s.vt_off + vs), p1 = __ldg(s.vt_off + ve);
-  const int q0 = __ldg(s.ee_once + es), q1 = __ldg(s.ee_once + ee);
+  const int q0 = __ldg(s.ee_off + es), q1 = __ldg(s.ee_off + ee);
   const int nv = p1 - p0, n = nv + (q1 - q0);
   R* ts = static_cast<R*>(s.ts);
   const R eps = R(s.eps), gamma = R(s.gamma);

@@ -10,7 +10,7 @@ namespace vbd {
 struct ScPersistentPlan {
   const int* inst_estart;  // [W+1] the edges of instance w are [inst_estart[w], inst_estart[w+1])
   const int* vt_off;       // [V+1] VT pairs of vertex v: vt_pairs[vt_off[v] .. vt_off[v+1])
-  const int* ee_once;      // [E+1] EE pairs of edge e that are no mirrors: ee_pairs[ee_once[e] .. ee_once[e+1])
+  const int* ee_off;       // [E+1] EE pairs of edge e: ee_pairs[ee_off[e] .. ee_off[e+1])
   const int4* vt_pairs;    // per pair its four vertices (ScBuffers::vt_pairs, ee_pairs)
   const int4* ee_pairs;
   void* ts;                // [V] R: per-vertex step fractions of the truncation, 1 between passes
