@@ -658,6 +658,19 @@ RingView ring_view(const VbdSolver* h) {
 template <typename T>
 int upload(T** d, const std::vector<T>& h);
 
+// Allows fn's launches all the dynamic shared memory that its static part leaves. The limit belongs to the function, which
+// every solver of the process on this device shares: one set to a solver's own size refuses the launches of a larger
+// solver that is still alive.
+int allow_shared(const void* fn) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes a;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  CK(cudaFuncGetAttributes(&a, fn));
+  CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - int(a.sharedSizeBytes)));
+  return VBD_OK;
+}
+
 // The records of the split-instance plan from the model's current materials, into the buffers that are there when
 // their sizes are the same (a captured graph keeps reading them).
 template <typename T>
@@ -812,7 +825,7 @@ int build_parts(VbdSolver* h, const std::vector<int>& wstart) {
   // a refresh may bring hinge damping: both variants have to fit
   const void* fns[2] = {parts_kernel(h, false), parts_kernel(h, true)};
   for (const void* fn : fns) {
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(g.smem)));
+    if ((rc = allow_shared(fn))) return rc;
     if (!g.grid && g.P > 8) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   }
   int fit = 1 << 30;
@@ -1647,7 +1660,10 @@ int occupancy_grid(VbdSolver* h) {
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const size_t dyn = h->smem_bytes;
-  if (dyn > 0) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
+  if (dyn > 0) {
+    const int rc = allow_shared(fn);
+    if (rc) return rc;
+  }
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, h->block, dyn));
   if (per_sm < 1) return VBD_ERR_INVALID_ARGUMENT;
   const int per_cta = h->warp_inst ? h->block / 32 : 1;  // instances a CTA works on at once
