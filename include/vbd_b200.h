@@ -132,6 +132,8 @@ typedef struct VbdSolverParams {
                                    instances from the work queue on its own (colors separated by __syncwarp, eight
                                    instances side by side in a CTA of 256; positions in shared memory per warp when
                                    they fit), for batches of small instances; 0 = one instance per CTA */
+  int32_t split;                /* 0 = cloths may run split over several CTAs each (see vbd_get_split), 1 = never: the
+                                   kernel that schedule, layout and the launch shape name */
 } VbdSolverParams;
 
 typedef struct VbdContactsDesc {
@@ -220,6 +222,14 @@ int vbd_launches_per_step(VbdHandle h, int32_t* out);
    be NULL. */
 int vbd_get_config(VbdHandle h, int32_t* schedule, int32_t* lanes_per_vertex, int32_t* block_size,
                    int32_t* shared_bytes, int32_t* layout);
+
+/* Split instances. A cloth-only model of fewer than six worlds per SM, 2 to 32 colors and at least one iteration whose
+   options are the defaults, or whose layout is ELL16 (AUTO or PERSISTENT schedule, any launch shape, not paired, not
+   per warp), steps in one launch of another kernel that sweeps every instance with several CTAs; the options then name
+   what runs with split = 1. parts: CTAs per job, jobs: runs of whole worlds that are swept one after the other, lanes
+   per vertex, threads per CTA, grid: 1 when the CTAs are a cooperative grid, 0 when they are one cluster. All 0 when the
+   handle steps unsplit. Any pointer may be NULL. */
+int vbd_get_split(VbdHandle h, int32_t* parts, int32_t* jobs, int32_t* lanes, int32_t* threads, int32_t* grid);
 
 int vbd_destroy(VbdHandle h);
 

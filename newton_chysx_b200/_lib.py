@@ -67,7 +67,7 @@ class VbdSolverParams(C.Structure):
         ("schedule", C.c_int32), ("lanes_per_vertex", C.c_int32), ("block_size", C.c_int32),
         ("contact_slots", C.c_int32), ("positions_in_shared", C.c_int32), ("layout", C.c_int32),
         ("min_blocks_per_sm", C.c_int32), ("pair_vertices", C.c_int32),
-        ("instance_per_warp", C.c_int32),
+        ("instance_per_warp", C.c_int32), ("split", C.c_int32),
     ]  # fmt: skip
 
 
@@ -130,6 +130,7 @@ SIGNATURES = {
     "vbd_get_residuals": ([_vp, _dp, C.c_int32, _vp], C.c_int),
     "vbd_launches_per_step": ([_vp, _ip], C.c_int),
     "vbd_get_config": ([_vp, _ip, _ip, _ip, _ip, _ip], C.c_int),
+    "vbd_get_split": ([_vp, _ip, _ip, _ip, _ip, _ip], C.c_int),
     "vbd_destroy": ([_vp], C.c_int),
     "vbd_color_particles": (
         [C.c_int32, C.c_int32, _ip, _fp, C.c_int32, _ip, _fp, C.c_int32, C.c_float, _ip],

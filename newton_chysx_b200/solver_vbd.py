@@ -24,8 +24,10 @@ Beyond the reference keywords:
   256 threads per SM (a register budget); 0 leaves the compiler's choice.
 * ``pair_vertices``: the ell16 persistent kernel (FP32) solves two vertices per thread, one in each lane
   of Blackwell's paired FP32 instructions (FFMA2 / FADD2 / FMUL2), halving the arithmetic instructions.
-* Cloths with default options, and ell16 batches of fewer than six worlds per SM, run split over several CTAs each
-  (one launch per substep); ``schedule``, ``layout`` and ``lanes_per_vertex`` then name what they would take unsplit.
+* ``split``: ``"auto"`` runs cloths of fewer than six worlds per SM split over several CTAs each (one launch per
+  substep) when the options are the defaults or the layout is ``"ell16"``, whatever the launch shape; ``"off"`` keeps
+  the kernel that ``schedule``, ``layout`` and the launch shape name. ``solver.split`` tells which one steps. A split
+  takes the whole GPU: several solvers that step at the same time on their own streams may do better without.
 * ``instance_per_warp``: the persistent csr kernel gives each warp its own instance (colors separated by
   ``__syncwarp`` instead of a CTA barrier), for batches of small instances such as soft-body blocks.
 
@@ -136,6 +138,7 @@ class SolverVBD:
         min_blocks_per_sm: int = 0,
         pair_vertices: bool = False,
         instance_per_warp: bool = False,
+        split: str = "auto",
     ):
         if rigid_avbd_beta < 0:
             raise ValueError(f"rigid_avbd_beta must be >= 0, got {rigid_avbd_beta}")
@@ -271,6 +274,7 @@ class SolverVBD:
         prm.min_blocks_per_sm = int(min_blocks_per_sm)
         prm.pair_vertices = int(bool(pair_vertices))
         prm.instance_per_warp = int(bool(instance_per_warp))
+        prm.split = {"auto": 0, "off": 1}[split]
         self._prm = prm
 
         h = C.c_void_p()
@@ -383,6 +387,16 @@ class SolverVBD:
         """The reference registers rigid-body Dahl-friction attributes here; cloth needs none."""
 
     # ------------------------------------------------------------------ diagnostics
+    @property
+    def split(self) -> dict | None:
+        """How the step's instances are split (``parts`` CTAs per job, ``jobs``, ``lanes`` per vertex, ``threads`` per
+        CTA, ``grid``: a cooperative grid instead of one cluster), or None when the kernel that ``schedule``, ``layout``,
+        ``lanes_per_vertex``, ``block_size`` and ``shared_bytes`` name steps them."""
+        n = [C.c_int32() for _ in range(5)]
+        _lib.check(self._lib.vbd_get_split(self._h, *(C.byref(x) for x in n)), "vbd_get_split")
+        parts, jobs, lanes, threads, grid = (x.value for x in n)
+        return dict(parts=parts, jobs=jobs, lanes=lanes, threads=threads, grid=bool(grid)) if parts else None
+
     def device_errors(self) -> int:
         bits = C.c_int32()
         stream = self._stream()

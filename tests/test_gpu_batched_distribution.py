@@ -3,7 +3,7 @@
 The batched benchmark steps 4,096 cloth instances whose grid sides are drawn from 16..128 vertices, with
 Young's moduli log-uniform in [1e3, 1e6] Pa, bending stiffness log-uniform in [1e-5, 1e-3] and one to four
 pinned corners, over a ground plane, through the 16-bit stencil persistent kernel. These tests run that
-kernel, in each launch shape the autotuner chooses from, on a batch spanning the same ranges (sides 16, 37,
+kernel, in each launch shape the autotuner chooses from, and the split that smaller batches take, on a batch spanning the same ranges (sides 16, 37,
 64, 101 and 128, each at both ends of the modulus and bending ranges), half of the instances falling freely
 and half pressed 0.5 mm into the ground, and compare every substep with the FP64 oracle (the CPU restatement
 of the reference step): from the same FP32 input, and along the trajectory. Tolerance: 1e-4 m (the cloth
@@ -25,9 +25,10 @@ DT = 1.0 / 600.0
 TOL = 1e-4
 
 SHAPES = {
-    "occ3": dict(layout="ell16", min_blocks_per_sm=3),
-    "occ4": dict(layout="ell16", min_blocks_per_sm=4),
-    "occ2": dict(layout="ell16", min_blocks_per_sm=2),
+    "occ3": dict(layout="ell16", min_blocks_per_sm=3, split="off"),
+    "occ4": dict(layout="ell16", min_blocks_per_sm=4, split="off"),
+    "occ2": dict(layout="ell16", min_blocks_per_sm=2, split="off"),
+    "split": dict(layout="ell16", min_blocks_per_sm=3),
     "paired": dict(layout="ell16", pair_vertices=True),
 }
 
@@ -81,7 +82,7 @@ def test_benchmark_distribution_matches_fp64_oracle(batch, shape):
     model, oracle_step, traj64, contacts = batch
     assert min(contacts) > 0  # the pressed instances are in contact throughout
     solver = SolverVBD(model, iterations=10, schedule="persistent", **SHAPES[shape])
-    assert solver.layout == "ell16" and solver.schedule == "persistent"
+    assert solver.layout == "ell16" and solver.schedule == "persistent" and (solver.split is not None) == (shape == "split")
     pipe = CollisionPipeline(model, soft_contact_margin=0.01)
     c = pipe.contacts()
     s0, s1 = model.state(), model.state()

@@ -150,9 +150,10 @@ def test_shape_table_limit():
     assert rc == _lib.VBD_ERR_UNSUPPORTED
 
 
-@pytest.mark.parametrize("layout,schedule", [("csr", "per_color"), ("ell", "per_color"), ("ell", "persistent"),
-                                             ("ell16", "persistent")])  # fmt: skip
-def test_sliver_triangles_match_oracle(layout, schedule):
+@pytest.mark.parametrize("layout,schedule,split", [("csr", "per_color", "off"), ("ell", "per_color", "off"),
+                                                   ("ell", "persistent", "off"), ("ell16", "persistent", "off"),
+                                                   ("ell16", "persistent", "auto")])  # fmt: skip
+def test_sliver_triangles_match_oracle(layout, schedule, split):
     """Triangles whose rest area is ~1e-6 of nominal (the precision stress sheet at 16 x 16): the stencil records
     carry mu and lambda times the area, which for slivers falls below the 1e-6 floor the reference applies to
     |lambda + mu|; the floor must act on the material values, as in the reference. FP64 against the FP64 oracle
@@ -162,8 +163,8 @@ def test_sliver_triangles_match_oracle(layout, schedule):
     b, sites = bench.build_precision_model(n=16, seed=4, sliver_fraction=0.05)
     assert len(sites) > 0
     model = b.finalize("cuda")
-    solver = SolverVBD(model, iterations=5, precision="fp64", schedule=schedule, layout=layout)
-    assert solver.layout == layout
+    solver = SolverVBD(model, iterations=5, precision="fp64", schedule=schedule, layout=layout, split=split)
+    assert solver.layout == layout and (solver.split is not None) == (split == "auto")
     om = orc.Model(oracle_model_dict(model))
     q = model.particle_q.double().cpu().numpy()
     qd = np.zeros_like(q)

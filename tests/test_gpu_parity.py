@@ -20,12 +20,13 @@ pytestmark = pytest.mark.gpu
 
 # step_grid_bodies: shapes on two bodies moved by an external rigid solver (integrate_with_external_rigid_solver)
 FIXTURES = ["step_grid_ground.npz", "step_grid_sphere.npz", "step_complex_rest_angle.npz", "step_grid_bodies.npz"]
-# (schedule, lanes per vertex, positions in shared memory, element layout)
+# (schedule, lanes per vertex, positions in shared memory, element layout); (persistent, 1, auto, ell16)
+# steps split over CTAs, the others do not
 LAUNCH = [("per_color", 1, "auto", "ell"), ("per_color", 1, "auto", "csr"), ("per_color", 4, "auto", "csr"),
           ("persistent", 1, "on", "ell"), ("persistent", 1, "off", "ell"), ("persistent", 1, "on", "csr"),
           ("persistent", 8, "on", "csr"), ("persistent", 32, "on", "csr"), ("persistent", 4, "off", "csr"),
           ("persistent", 1, "on", "ell16"), ("persistent", 1, "off", "ell16"), ("persistent", 1, "on", "ring"),
-          ("persistent", 1, "off", "ring")]
+          ("persistent", 1, "off", "ring"), ("persistent", 1, "auto", "ell16")]
 
 
 def _state(arr, dtype=torch.float32):
@@ -51,11 +52,14 @@ def _run_golden_substep(solver, g, s, dtype=torch.float32):
 def test_fp32_step_matches_reference_goldens(name, schedule, lanes, shared, layout):
     g = load_golden(name)
     model = model_from_golden(g)
+    split = (schedule, shared) == ("persistent", "auto")
     solver = SolverVBD(model, iterations=int(g["iterations"]), friction_epsilon=float(g["friction_epsilon"]),
                        rigid_avbd_beta=float(g["beta"]), schedule=schedule, lanes_per_vertex=lanes,
-                       positions_in_shared=shared, layout=layout, **golden_solver_kw(g))  # fmt: skip
+                       positions_in_shared=shared, layout=layout, split="auto" if split else "off",
+                       **golden_solver_kw(g))  # fmt: skip
     assert solver.schedule == schedule and solver.lanes_per_vertex == lanes and solver.layout == layout
-    assert (solver.shared_bytes > 0) == (schedule == "persistent" and shared == "on")
+    assert (solver.shared_bytes > 0) == (schedule == "persistent" and shared != "off")
+    assert (solver.split is not None) == split
     for s in range(int(g["substeps"])):
         st_in, st_out = _run_golden_substep(solver, g, s)
         q_out = st_out.particle_q.cpu().numpy()
@@ -78,7 +82,7 @@ def test_paired_vertices_match_reference_goldens(occ, shared):
     model = model_from_golden(g)
     kw = dict(iterations=int(g["iterations"]), friction_epsilon=float(g["friction_epsilon"]),
               rigid_avbd_beta=float(g["beta"]), schedule="persistent", layout="ell16", positions_in_shared=shared,
-              min_blocks_per_sm=occ)  # fmt: skip
+              min_blocks_per_sm=occ, split="off")  # fmt: skip
     paired = SolverVBD(model, pair_vertices=True, **kw)
     plain = SolverVBD(model, **kw)
     for s in range(int(g["substeps"])):
@@ -103,7 +107,8 @@ def test_paired_vertices_on_a_batch(occ):
     mats[5, :2] = 0.0  # one triangle with mu = lambda = 0 (skipped by the sweep)
     b._tri_mat = [mats]
     model = b.finalize("cuda")
-    kw = dict(iterations=10, schedule="persistent", layout="ell16", positions_in_shared="off", min_blocks_per_sm=occ)
+    kw = dict(iterations=10, schedule="persistent", layout="ell16", positions_in_shared="off", min_blocks_per_sm=occ,
+              split="off")  # fmt: skip
     paired, plain = SolverVBD(model, pair_vertices=True, **kw), SolverVBD(model, **kw)
     pipe = sim.CollisionPipeline(model, soft_contact_margin=0.01)
     contacts = pipe.contacts()
@@ -135,9 +140,11 @@ def test_paired_vertices_need_fp32_ell16_persistent():
 
 
 @pytest.mark.parametrize("name", FIXTURES)
-@pytest.mark.parametrize("schedule,layout", [("per_color", "ell"), ("per_color", "csr"), ("persistent", "ell"),
-                                             ("persistent", "csr"), ("persistent", "ell16"), ("persistent", "ring")])
-def test_fp64_step_matches_fp64_oracle(name, schedule, layout):
+@pytest.mark.parametrize("schedule,layout,split", [("per_color", "ell", "off"), ("per_color", "csr", "off"),
+                                                   ("persistent", "ell", "off"), ("persistent", "csr", "off"),
+                                                   ("persistent", "ell16", "off"), ("persistent", "ring", "off"),
+                                                   ("persistent", "ell16", "auto")])  # fmt: skip
+def test_fp64_step_matches_fp64_oracle(name, schedule, layout, split):
     """Every layout in FP64 against the FP64 oracle; step_grid_ground and step_complex_rest_angle carry hinge
     damping, which the 16-bit stencil layout reads from its side array and the one-ring layout evaluates per
     damped hinge."""
@@ -145,7 +152,8 @@ def test_fp64_step_matches_fp64_oracle(name, schedule, layout):
     model = model_from_golden(g)
     solver = SolverVBD(model, iterations=int(g["iterations"]), friction_epsilon=float(g["friction_epsilon"]),
                        rigid_avbd_beta=float(g["beta"]), precision="fp64", schedule=schedule, layout=layout,
-                       **golden_solver_kw(g))  # fmt: skip
+                       split=split, **golden_solver_kw(g))  # fmt: skip
+    assert (solver.split is not None) == (split == "auto")
     om = orc.Model(oracle_model_dict(model, float(g["friction_epsilon"]), float(g["beta"])))
     for s in range(int(g["substeps"])):
         st_in, st_out = _run_golden_substep(solver, g, s, torch.float64)

@@ -301,7 +301,8 @@ def test_schedules_and_lane_counts_agree():
                                             ("persistent", 1, "off", "ell16"), ("persistent", 1, "on", "ring"),
                                             ("persistent", 1, "off", "ring")]:
         solver = SolverVBD(model, iterations=10, schedule=schedule, lanes_per_vertex=lanes, positions_in_shared=shared,
-                           layout=layout)  # fmt: skip
+                           layout=layout, split="off")  # fmt: skip
+        assert solver.split is None
         s = _run(model, solver, 3, 10, 1.0 / 600.0, CollisionPipeline(model))
         results.append(s.particle_q.cpu().numpy())
     for r in results[1:]:
@@ -323,11 +324,11 @@ def test_batched_worlds_match_single_instances():
     assert solver.shared_bytes == 12 * max(n * n for n in sizes)
     s = _run(model, solver, 2, 10, 1.0 / 600.0)
     q = s.particle_q.cpu().numpy()
-    assert solver.layout == "ell16"
+    assert solver.layout == "ell16" and solver.split is not None
     for shared, layout in [("off", "ell"), ("on", "csr"), ("off", "csr"), ("off", "ell16"), ("off", "ring"),
                            ("on", "ring")]:
         s_g = _run(model, SolverVBD(model, iterations=10, schedule="persistent", positions_in_shared=shared,
-                                    layout=layout), 2, 10, 1.0 / 600.0)  # fmt: skip
+                                    layout=layout, split="off"), 2, 10, 1.0 / 600.0)  # fmt: skip
         assert np.abs(s_g.particle_q.cpu().numpy() - q).max() <= 1e-5
     start = 0
     for b in singles:

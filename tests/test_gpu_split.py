@@ -68,11 +68,15 @@ def _run(model, q, qd, substeps=2, **kw):
 
 
 # 9 x 7: less than two CTAs' worth; 32 x 32: the largest cluster; 41 x 27: the first grid; 300 x 60: 148 CTAs with
-# eight lanes; 256 x 97 and 411 x 260: four and two lanes; 700 x 801: runs longer than a CTA's threads
-@pytest.mark.parametrize("nx,ny,kd,shapes", [(9, 7, 0.0, 1), (32, 32, 1e-3, 3), (41, 27, 0.0, 2), (300, 60, 1e-3, 1),
-                                              (256, 97, 0.0, 1), (411, 260, 0.0, 1), (700, 801, 0.0, 1)])  # fmt: skip
-def test_split_sheet_matches_the_per_color_kernels(nx, ny, kd, shapes):
+# eight lanes; 320 x 160 and 411 x 260: four and two lanes; 700 x 801: one lane, runs longer than a CTA's threads
+@pytest.mark.parametrize("nx,ny,kd,shapes,parts,lanes,grid", [
+    (9, 7, 0.0, 1, 2, 8, False), (32, 32, 1e-3, 3, 16, 8, False), (41, 27, 0.0, 2, 18, 8, True),
+    (300, 60, 1e-3, 1, 148, 8, True), (320, 160, 0.0, 1, 148, 4, True), (411, 260, 0.0, 1, 148, 2, True),
+    (700, 801, 0.0, 1, 148, 1, True)])  # fmt: skip
+def test_split_sheet_matches_the_per_color_kernels(nx, ny, kd, shapes, parts, lanes, grid):
     model = _sheet(nx, ny, kd, shapes).finalize("cuda:0")
+    chosen = SolverVBD(model, iterations=6).split
+    assert (chosen["parts"], chosen["lanes"], chosen["grid"], chosen["jobs"]) == (parts, lanes, grid, 1)
     model.soft_contact_ke, model.soft_contact_kd, model.soft_contact_mu = 1e4, 1e-4, 0.5
     q, qd = _start(model, nx)
     ref, ref_d = _run(model, q, qd, precision="fp64", schedule="per_color")
@@ -95,6 +99,8 @@ def test_split_worlds_match_the_one_cta_kernel(sides):
     model.soft_contact_ke, model.soft_contact_kd, model.soft_contact_mu = 1e4, 1e-4, 0.5
     q, qd = _start(model, len(sides))
     ref, _ = _run(model, q, qd, precision="fp64", schedule="persistent", layout="ell")
+    chosen = SolverVBD(model, iterations=6, schedule="persistent", layout="ell16", min_blocks_per_sm=3).split
+    assert chosen["grid"] == (len(q) > 1024)
     got, _ = _run(model, q, qd, precision="fp64", schedule="persistent", layout="ell16")
     assert np.abs(got - ref).max() <= 1e-9
     got, _ = _run(model, q, qd, substeps=1, schedule="persistent", layout="ell16", min_blocks_per_sm=3)
@@ -147,9 +153,29 @@ def test_split_refresh_and_capture(n):
     del graph
 
 
-def test_split_leaves_explicit_shapes_and_small_models_alone():
-    b = cloth_grid_builder(n=12)
-    model = b.finalize("cuda:0")
-    assert SolverVBD(model, iterations=4, schedule="per_color").launches_per_step > 4
-    assert SolverVBD(model, iterations=4).launches_per_step <= 2
-    assert SolverVBD(model, iterations=0).launches_per_step <= 2
+def test_what_steps_split_and_what_does_not():
+    """The split is reported, taken with the default options and with ell16 whatever its launch shape, and left where an
+    option names another kernel, split="off" asks for it, there is nothing to split or enough worlds fill the GPU."""
+    model = cloth_grid_builder(n=12).finalize("cuda:0")
+    small = dict(parts=3, jobs=1, lanes=8, grid=False)
+    for kw in ({}, dict(schedule="persistent"), dict(precision="mixed"), dict(precision="fp64"), dict(layout="ell16", schedule="persistent"),
+               dict(layout="ell16", schedule="persistent", lanes_per_vertex=1, block_size=128, min_blocks_per_sm=3,
+                    positions_in_shared="off")):  # fmt: skip
+        got = SolverVBD(model, iterations=4, **kw).split
+        assert got is not None and {k: got[k] for k in small} == small and got["threads"] >= 64
+    ell16 = dict(layout="ell16", schedule="persistent")
+    for kw in (dict(split="off"), dict(ell16, split="off"), dict(schedule="per_color"), dict(layout="csr"), dict(layout="ell"),
+               dict(layout="ring", schedule="persistent"), dict(block_size=128), dict(lanes_per_vertex=4),
+               dict(positions_in_shared="on"), dict(ell16, pair_vertices=True), dict(iterations=0),
+               dict(particle_enable_self_contact=True, particle_self_contact_radius=1e-3, particle_self_contact_margin=2e-3),
+               dict(layout="csr", schedule="persistent", lanes_per_vertex=4, instance_per_warp=True)):  # fmt: skip
+        assert SolverVBD(model, **dict(dict(iterations=4), **kw)).split is None, kw
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for worlds in (6 * sms - 1, 6 * sms):
+        top = nb.ModelBuilder(up_axis="Z", gravity=-9.81)
+        one = cloth_grid_builder(n=4)
+        for _ in range(worlds):
+            top.add_world(one)
+        assert (SolverVBD(top.finalize("cuda:0"), iterations=4).split is not None) == (worlds < 6 * sms)
+    with pytest.raises(KeyError):
+        SolverVBD(model, split="on")
