@@ -78,7 +78,7 @@ struct PartsPlan {
 };
 
 // Cuts the jobs (job_v0: first particle of each job, then V) into P parts each. False: the plan does not exist
-// (a part with 65,536 places or more, or an element that names a vertex twice, whose role the records cannot tell).
+// (a part with 65,536 places or more, or an element with two vertices of one color).
 bool parts_plan(const PartsInput& in, const std::vector<int>& job_v0, int P, int L, PartsPlan& plan);
 // The records of the plan's elements with the input's materials; kd stays empty when no hinge is damped.
 void parts_records(const PartsInput& in, const PartsPlan& plan, bool hinge_damping, std::vector<uint4>& faceA,

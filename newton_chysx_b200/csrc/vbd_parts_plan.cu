@@ -50,14 +50,21 @@ void neighbours(const PartsInput& in, int v, F f) {
 
 bool parts_plan(const PartsInput& in, const std::vector<int>& job_v0, int P, int L, PartsPlan& plan) {
   const int V = in.V, C = in.C;
-  for (int t = 0; t < in.T; ++t) {
-    const int* x = in.tri + 3 * size_t(t);
-    if (x[0] == x[1] || x[0] == x[2] || x[1] == x[2]) return false;
-  }
+  // Vertices of an element in one color (a coloring without the hinges leaves opposite vertices so) would break the flags'
+  // argument in vbd_parts.cu; whatever the element's stiffness, which a refresh can switch on. Also rules out an element
+  // that names a vertex twice.
+  const auto apart = [&](const int* x, int n) {
+    for (int i = 0; i < n; ++i)
+      for (int j = 0; j < i; ++j)
+        if (in.color_of[x[i]] == in.color_of[x[j]]) return false;
+    return true;
+  };
+  for (int t = 0; t < in.T; ++t)
+    if (!apart(in.tri + 3 * size_t(t), 3)) return false;
   for (int e = 0; e < in.E; ++e) {
     const int* x = in.edges + 4 * size_t(e);
     if (x[0] < 0 || x[1] < 0) continue;  // a boundary hinge: no record
-    if (x[0] == x[1] || x[0] == x[2] || x[0] == x[3] || x[1] == x[2] || x[1] == x[3] || x[2] == x[3]) return false;
+    if (!apart(x, 4)) return false;
   }
   plan = PartsPlan();
   plan.P = P, plan.L = L, plan.C = C;

@@ -170,6 +170,22 @@ def test_what_steps_split_and_what_does_not():
                dict(particle_enable_self_contact=True, particle_self_contact_radius=1e-3, particle_self_contact_margin=2e-3),
                dict(layout="csr", schedule="persistent", lanes_per_vertex=4, instance_per_warp=True)):  # fmt: skip
         assert SolverVBD(model, **dict(dict(iterations=4), **kw)).split is None, kw
+    # vertices of an element in one color: opposite vertices of a hinge with the default coloring, and of a triangle
+    # without stiffness, which a refresh can switch on
+    for triangles in (False, True):
+        b = cloth_grid_builder(n=12)
+        if triangles:
+            free = int(b.tri_indices[-1][0])
+            groups = [[int(v) for v in g if int(v) != free] for g in b.particle_color_groups]
+            other = int(b.tri_indices[-1][1])
+            next(g for g in groups if other in g).append(free)
+            mats = b.tri_materials
+            mats[(b.tri_indices == free).any(axis=1), :2] = 0.0
+            b._tri_mat = [mats]
+            b.set_coloring([np.sort(np.int32(g)) for g in groups])
+        else:
+            b.color()
+        assert SolverVBD(b.finalize("cuda:0"), iterations=4).split is None
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     for worlds in (6 * sms - 1, 6 * sms):
         top = nb.ModelBuilder(up_axis="Z", gravity=-9.81)
