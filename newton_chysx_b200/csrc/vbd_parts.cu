@@ -385,8 +385,15 @@ __global__ void __launch_bounds__(T, 1)
         }
       }
     // the damping terms read ghosts' start positions from state_in: their owners write it back when all have finished
-    if (grid_mode && (HD || p.face_damping))
-      for (int g = g0 + tid; g < g1; g += nt) wait_done(p.done + __ldg(p.ghost_part + g) * kDoneStride, phase);
+    if (grid_mode && (HD || p.face_damping)) {
+      for (int g = g0 + tid; g < g1; g += nt)
+        if (!wait_done(p.done + __ldg(p.ghost_part + g) * kDoneStride, phase)) s_abort = 1;
+      __syncthreads();
+      if (s_abort) {
+        if (tid == 0) set_err(c.err, kErrBarrier);
+        return;
+      }
+    }
     __syncthreads();
     for (int slot = tid; slot < nown; slot += nt) {
       const int v = __ldg(p.vert + v0 + slot) & 0x7fffffff;
