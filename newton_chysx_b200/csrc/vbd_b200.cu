@@ -231,13 +231,13 @@ struct VbdSolver {
   bool parts_on = false;
   PartsConfig parts;
   PartsPlan plan;
-  bool parts_damped = false, parts_face_damped = false;
   std::vector<int> color_of;  // [V] place of each particle's color in the sweep
   int* color_of_dev = nullptr;
   PartsView pt = {};
   char* pt_blob = nullptr;
   uint4 *pt_faceA = nullptr, *pt_faceB = nullptr, *pt_hinge = nullptr;
   float* pt_kd = nullptr;
+  int* pt_damping = nullptr;
   float4* pt_contact = nullptr;
   // adjoint work buffers (allocated by the first vbd_adjoint_step)
   void* adj_work = nullptr;
@@ -263,7 +263,7 @@ struct VbdSolver {
                   ell16_faceA, ell16_faceB, ell16_hinge, sc_pos_cd, sc_disp, sc_ts, ring_nslot, ring_base,
                   ring_vbase, ring_A, ring_B, ring_H, ring_hdr, ring_kd, spr_idx, spr_prop, spr_off, spr_adj, sspr_off,
                   sspr_adj, spr_acc, tet_idx, tet_pose, tet_off, tet_adj, sc_estart, sc_world, pt_blob, color_of_dev, live, pt_faceA, pt_faceB, pt_hinge,
-                  pt_kd, pt_contact};
+                  pt_kd, pt_damping, pt_contact};
     for (void* p : ps)
       if (p) cudaFree(p);
     sc_release(sc);
@@ -702,21 +702,21 @@ int parts_input(VbdSolver* h, PartsInput& in, std::vector<float> buf[6]) {
 }
 
 int upload_parts_records(VbdSolver* h, const PartsInput& in, bool have) {
-  bool damped = false, face_damped = false;
-  for (int e = 0; e < h->E; ++e) damped |= in.bending[2 * size_t(e)] > 0.f && in.bending[2 * size_t(e) + 1] > 0.f;
+  std::vector<int> damping = {0};
+  for (int e = 0; e < h->E; ++e)
+    if (in.bending[2 * size_t(e)] > 0.f && in.bending[2 * size_t(e) + 1] > 0.f) damping[0] |= kHingeDamping;
   for (int t = 0; t < h->T; ++t) {
     const float* m = in.mat + 5 * size_t(t);
-    face_damped |= (m[0] > 0.f || m[1] > 0.f) && m[2] > 0.f;
+    if ((m[0] > 0.f || m[1] > 0.f) && m[2] > 0.f) damping[0] |= kFaceDamping;
   }
   std::vector<uint4> fa, fb, hg;
   std::vector<float> kd;
-  parts_records(in, h->plan, damped, fa, fb, hg, kd);
+  parts_records(in, h->plan, fa, fb, hg, kd);
   int rc;
   if ((rc = upload_same(&h->pt_faceA, fa, have)) || (rc = upload_same(&h->pt_faceB, fb, have)) ||
-      (rc = upload_same(&h->pt_hinge, hg, have)) || (damped && (rc = upload_same(&h->pt_kd, kd, have))))
+      (rc = upload_same(&h->pt_hinge, hg, have)) || (rc = upload_same(&h->pt_kd, kd, have)) ||
+      (rc = upload_same(&h->pt_damping, damping, have)))
     return rc;
-  h->parts_damped = damped;
-  h->parts_face_damped = face_damped;
   return VBD_OK;
 }
 
@@ -748,18 +748,18 @@ PartsView parts_view(const VbdSolver* h) {
   p.C = h->plan.C, p.P = h->plan.P, p.njobs = h->plan.njobs;
   p.places = h->plan.most_places, p.most_own = h->plan.most_own;
   p.faceA = h->pt_faceA, p.faceB = h->pt_faceB, p.hinge = h->pt_hinge;
-  p.hinge_kd = h->parts_damped ? h->pt_kd : nullptr;
-  p.face_damping = h->parts_face_damped;
+  p.hinge_kd = h->pt_kd;
+  p.damping = h->pt_damping;
   p.contact = h->pt_contact;
   p.queue = h->queue;
   p.done = reinterpret_cast<unsigned*>(h->queue + kDoneStride);
   return p;
 }
 
-const void* parts_kernel(const VbdSolver* h, bool damped) {
-  if (h->precision == VBD_PRECISION_FP64) return parts_fn<double, MODE_FP64>(h->parts.L, false, damped);
-  if (h->precision == VBD_PRECISION_MIXED) return parts_fn<float, MODE_MIXED>(h->parts.L, h->parts.wide, damped);
-  return parts_fn<float, MODE_FP32>(h->parts.L, h->parts.wide, damped);
+const void* parts_kernel(const VbdSolver* h) {
+  if (h->precision == VBD_PRECISION_FP64) return parts_fn<double, MODE_FP64>(h->parts.L, false);
+  if (h->precision == VBD_PRECISION_MIXED) return parts_fn<float, MODE_MIXED>(h->parts.L, h->parts.wide);
+  return parts_fn<float, MODE_FP32>(h->parts.L, h->parts.wide);
 }
 
 // Decides whether instances are split (wstart: first particle of each world, then V) and builds the plan. Leaves
@@ -822,32 +822,25 @@ int build_parts(VbdSolver* h, const std::vector<int>& wstart) {
   g.smem = place * size_t(h->plan.most_places) + (place + sizeof(int)) * size_t(h->plan.most_own);
   if (g.smem + 2048 > size_t(optin)) return VBD_OK;
   h->parts = g;
-  // a refresh may bring hinge damping: both variants have to fit
-  const void* fns[2] = {parts_kernel(h, false), parts_kernel(h, true)};
-  for (const void* fn : fns) {
-    if ((rc = allow_shared(fn))) return rc;
-    if (!g.grid && g.P > 8) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  }
-  int fit = 1 << 30;
-  for (const void* fn : fns) {
-    int n = 0;
-    if (g.grid) {
-      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, g.block, g.smem));
-      n = n * sms / g.P;
-    } else {
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = g.P;
-      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(g.P);
-      cfg.blockDim = dim3(g.block);
-      cfg.dynamicSmemBytes = g.smem;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      CK(cudaOccupancyMaxActiveClusters(&n, fn, &cfg));
-    }
-    fit = std::min(fit, n);
+  const void* fn = parts_kernel(h);
+  if ((rc = allow_shared(fn))) return rc;
+  int fit = 0;
+  if (g.grid) {
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, g.block, g.smem));
+    fit = fit * sms / g.P;
+  } else {
+    if (g.P > 8) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = g.P;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(g.P);
+    cfg.blockDim = dim3(g.block);
+    cfg.dynamicSmemBytes = g.smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CK(cudaOccupancyMaxActiveClusters(&fit, fn, &cfg));
   }
   if (fit < 1) return VBD_OK;
   h->parts.blocks = g.P * (g.grid ? 1 : std::min(fit, h->plan.njobs));
@@ -1440,7 +1433,7 @@ int step_impl(VbdSolver* h, R* q_in, R* q_out, const R* qd_in, R* qd_out, const 
       CK(cudaMemsetAsync(h->slot_cnt, 0, sizeof(int) * h->V, st));
       k_contact_prepare<R><<<(c.c_max + 255) / 256, 256, 0, st>>>(c);
     }
-    CK((launch_parts<R, MODE>(h->parts, h->parts_damped, c, parts_view(h), iters, st)));
+    CK((launch_parts<R, MODE>(h->parts, c, parts_view(h), iters, st)));
   } else if (h->schedule == VBD_SCHEDULE_PERSISTENT) {
     CK(cudaMemsetAsync(h->queue, 0, sizeof(int), st));
     if (has_c) {

@@ -282,21 +282,74 @@ __device__ __forceinline__ void solve_part(const StepCtx<R>& c, const PartsView&
   if (code < 0) c.pos[v] = pk4(xn, R(0));
 }
 
+// The job's plan entries of this part in shared memory.
+struct PartShared {
+  int abort;
+  int start[kPartColors + 1], go[kPartColors + 1], nf[kPartColors], ne[kPartColors];
+  long long fb[kPartColors], eb[kPartColors];
+};
+
+// The iterations of one job. False: a wait ran out.
+template <typename R, int MODE, int L, bool HD, bool EARLY>
+__device__ __forceinline__ bool sweep_part(const StepCtx<R>& c, const PartsView& p, PartShared& s, pos4_t<R>* s_pos,
+                                           const pos4_t<R>* s_y, const int* s_kind, int v0, int nown, int g0,
+                                           const PartStart<R>& start, int rank, int grid_mode, int iterations,
+                                           unsigned& phase) {
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int group = tid / L, lane = tid % L, per_round = nt / L;
+  for (int it = 0; it < iterations; ++it)
+    for (int col = 0; col < p.C; ++col) {
+      const int a = s.start[col], n = s.start[col + 1] - a;
+      const int nf = s.nf[col], ne = s.ne[col];
+      const long long fb = s.fb[col], eb = s.eb[col];
+      const int gb = s.go[col], ge = s.go[col + 1];
+      int mine = 0, owner = 0;  // this thread's ghost, known before the wait
+      if (gb + tid < ge) mine = __ldg(p.ghost + gb + tid), owner = __ldg(p.ghost_part + gb + tid);
+      for (int base = 0; base < n; base += per_round) {
+        const int j = base + group;
+        const long long o = (long long)j * L + lane;
+        solve_part<R, MODE, L, HD, EARLY>(c, p, s_pos, s_y, s_kind, v0, start, a + j, j < n, lane, nf, ne,
+                                                     fb + o, eb + o, n * L, it);
+      }
+      if (p.P > 1) {
+        if (grid_mode) {
+          __syncthreads();
+          ++phase;
+          if (tid == 0) st_release(p.done + rank * kDoneStride, phase);
+          if (gb + tid < ge && !wait_done(p.done + owner * kDoneStride, phase)) s.abort = 1;
+        } else {
+          cluster_barrier();
+        }
+        if (gb + tid < ge) s_pos[nown + gb + tid - g0] = ld_l2(c.pos + mine);
+        for (int g = gb + tid + nt; g < ge; g += nt) {
+          if (grid_mode && !wait_done(p.done + __ldg(p.ghost_part + g) * kDoneStride, phase)) s.abort = 1;
+          s_pos[nown + g - g0] = ld_l2(c.pos + __ldg(p.ghost + g));
+        }
+      }
+      __syncthreads();
+      if (grid_mode && s.abort) {  // a wait ran out: report and leave
+        if (tid == 0) set_err(c.err, kErrBarrier);
+        return false;
+      }
+    }
+  return true;
+}
+
 // T: threads that the register budget allows, 512 (128 registers) for the latency of few vertices, 896 (72 registers)
 // where a part's colors have enough work to fill them, 384 in FP64.
-template <typename R, int MODE, int L, bool HD, int T>
+template <typename R, int MODE, int L, int T>
 __global__ void __launch_bounds__(T, 1)
     k_parts(const __grid_constant__ StepCtx<R> c, const __grid_constant__ PartsView p, int grid_mode, int iterations) {
   extern __shared__ __align__(32) unsigned char s_raw[];
   pos4_t<R>* s_pos = reinterpret_cast<pos4_t<R>*>(s_raw);
-  __shared__ int s_item, s_abort;
-  __shared__ int s_start[kPartColors + 1], s_go[kPartColors + 1], s_nf[kPartColors], s_ne[kPartColors];
-  __shared__ long long s_fb[kPartColors], s_eb[kPartColors];
+  __shared__ int s_item;
+  __shared__ PartShared s;
   namespace cg = cooperative_groups;
   const int rank = grid_mode ? int(blockIdx.x) : int(cg::this_cluster().block_rank());
   const int tid = threadIdx.x, nt = blockDim.x;
+  const int damping = *p.damping;
   unsigned phase = 0;
-  if (tid == 0) s_abort = 0;
+  if (tid == 0) s.abort = 0;
   for (int round = 0;; ++round) {
     int job = 0;
     if (grid_mode) {
@@ -321,13 +374,13 @@ __global__ void __launch_bounds__(T, 1)
     pos4_t<R>* s_y = s_pos + p.places;
     int* s_kind = reinterpret_cast<int*>(s_y + p.most_own);
     if (tid <= p.C) {
-      s_go[tid] = __ldg(go + tid);
-      s_start[tid] = __ldg(p.start + part * (p.C + 1) + tid);
+      s.go[tid] = __ldg(go + tid);
+      s.start[tid] = __ldg(p.start + part * (p.C + 1) + tid);
       if (tid < p.C) {
-        s_nf[tid] = __ldg(p.nf + part * p.C + tid);
-        s_ne[tid] = __ldg(p.ne + part * p.C + tid);
-        s_fb[tid] = __ldg(p.fbase + part * p.C + tid);
-        s_eb[tid] = __ldg(p.ebase + part * p.C + tid);
+        s.nf[tid] = __ldg(p.nf + part * p.C + tid);
+        s.ne[tid] = __ldg(p.ne + part * p.C + tid);
+        s.fb[tid] = __ldg(p.fbase + part * p.C + tid);
+        s.eb[tid] = __ldg(p.ebase + part * p.C + tid);
       }
     }
     for (int slot = tid; slot < nown; slot += nt) {
@@ -348,48 +401,21 @@ __global__ void __launch_bounds__(T, 1)
         s_pos[nown + g - g0] = pk4(predict(c, __ldg(p.ghost + g), q, ms), R(0));
       }
     __syncthreads();
-    const int group = tid / L, lane = tid % L, per_round = nt / L;
-    for (int it = 0; it < iterations; ++it)
-      for (int col = 0; col < p.C; ++col) {
-        const int a = s_start[col], n = s_start[col + 1] - a;
-        const int nf = s_nf[col], ne = s_ne[col];
-        const long long fb = s_fb[col], eb = s_eb[col];
-        const int gb = s_go[col], ge = s_go[col + 1];
-        int mine = 0, owner = 0;  // this thread's ghost, known before the wait
-        if (gb + tid < ge) mine = __ldg(p.ghost + gb + tid), owner = __ldg(p.ghost_part + gb + tid);
-        for (int base = 0; base < n; base += per_round) {
-          const int j = base + group;
-          const long long o = (long long)j * L + lane;
-          solve_part<R, MODE, L, HD, (T <= 512)>(c, p, s_pos, s_y, s_kind, v0, start, a + j, j < n, lane, nf, ne, fb + o,
-                                                 eb + o, n * L, it);
-        }
-        if (p.P > 1) {
-          if (grid_mode) {
-            __syncthreads();
-            ++phase;
-            if (tid == 0) st_release(p.done + rank * kDoneStride, phase);
-            if (gb + tid < ge && !wait_done(p.done + owner * kDoneStride, phase)) s_abort = 1;
-          } else {
-            cluster_barrier();
-          }
-          if (gb + tid < ge) s_pos[nown + gb + tid - g0] = ld_l2(c.pos + mine);
-          for (int g = gb + tid + nt; g < ge; g += nt) {
-            if (grid_mode && !wait_done(p.done + __ldg(p.ghost_part + g) * kDoneStride, phase)) s_abort = 1;
-            s_pos[nown + g - g0] = ld_l2(c.pos + __ldg(p.ghost + g));
-          }
-        }
-        __syncthreads();
-        if (grid_mode && s_abort) {  // a wait ran out: report and leave
-          if (tid == 0) set_err(c.err, kErrBarrier);
-          return;
-        }
-      }
+    // one sweep for each answer to whether hinges are damped: deciding per hinge took 5 % (32 x 32, 256 x 256) to 13 %
+    // (512 worlds) of an undamped step, this 1 (512 x 512) to 3 % (32 x 32: 4 us) against a kernel of its own for each,
+    // between which a captured step could not change
+    const bool done = damping & kHingeDamping
+                          ? sweep_part<R, MODE, L, true, (T <= 512)>(c, p, s, s_pos, s_y, s_kind, v0, nown, g0, start,
+                                                                     rank, grid_mode, iterations, phase)
+                          : sweep_part<R, MODE, L, false, (T <= 512)>(c, p, s, s_pos, s_y, s_kind, v0, nown, g0, start,
+                                                                      rank, grid_mode, iterations, phase);
+    if (!done) return;
     // the damping terms read ghosts' start positions from state_in: their owners write it back when all have finished
-    if (grid_mode && (HD || p.face_damping)) {
+    if (grid_mode && damping) {
       for (int g = g0 + tid; g < g1; g += nt)
-        if (!wait_done(p.done + __ldg(p.ghost_part + g) * kDoneStride, phase)) s_abort = 1;
+        if (!wait_done(p.done + __ldg(p.ghost_part + g) * kDoneStride, phase)) s.abort = 1;
       __syncthreads();
-      if (s_abort) {
+      if (s.abort) {
         if (tid == 0) set_err(c.err, kErrBarrier);
         return;
       }
@@ -406,30 +432,24 @@ __global__ void __launch_bounds__(T, 1)
   }
 }
 
-template <typename R, int MODE, bool HD>
-const void* parts_fn_l(int L, bool wide) {
-  if constexpr (sizeof(R) == 4) {
-    if (wide) return L == 1 ? (const void*)k_parts<R, MODE, 1, HD, 896> : (const void*)k_parts<R, MODE, 2, HD, 896>;
-  }
-  constexpr int T = sizeof(R) == 4 ? 512 : 384;
-  switch (L) {
-    case 1: return (const void*)k_parts<R, MODE, 1, HD, T>;
-    case 2: return (const void*)k_parts<R, MODE, 2, HD, T>;
-    case 4: return (const void*)k_parts<R, MODE, 4, HD, T>;
-    default: return (const void*)k_parts<R, MODE, 8, HD, T>;
-  }
-}
-
 }  // namespace
 
 template <typename R, int MODE>
-const void* parts_fn(int L, bool wide, bool damped) {
-  return damped ? parts_fn_l<R, MODE, true>(L, wide) : parts_fn_l<R, MODE, false>(L, wide);
+const void* parts_fn(int L, bool wide) {
+  if constexpr (sizeof(R) == 4) {
+    if (wide) return L == 1 ? (const void*)k_parts<R, MODE, 1, 896> : (const void*)k_parts<R, MODE, 2, 896>;
+  }
+  constexpr int T = sizeof(R) == 4 ? 512 : 384;
+  switch (L) {
+    case 1: return (const void*)k_parts<R, MODE, 1, T>;
+    case 2: return (const void*)k_parts<R, MODE, 2, T>;
+    case 4: return (const void*)k_parts<R, MODE, 4, T>;
+    default: return (const void*)k_parts<R, MODE, 8, T>;
+  }
 }
 
 template <typename R, int MODE>
-cudaError_t launch_parts(const PartsConfig& g, bool damped, const StepCtx<R>& c, const PartsView& p, int iterations,
-                         cudaStream_t st) {
+cudaError_t launch_parts(const PartsConfig& g, const StepCtx<R>& c, const PartsView& p, int iterations, cudaStream_t st) {
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g.blocks);
@@ -448,13 +468,12 @@ cudaError_t launch_parts(const PartsConfig& g, bool damped, const StepCtx<R>& c,
   }
   int grid_mode = g.grid ? 1 : 0;
   void* args[] = {(void*)&c, (void*)&p, (void*)&grid_mode, (void*)&iterations};
-  return cudaLaunchKernelExC(&cfg, parts_fn<R, MODE>(g.L, g.wide, damped), args);
+  return cudaLaunchKernelExC(&cfg, parts_fn<R, MODE>(g.L, g.wide), args);
 }
 
 #define VBD_PARTS(R, MODE)                                                                                       \
-  template const void* parts_fn<R, MODE>(int, bool, bool);                                                      \
-  template cudaError_t launch_parts<R, MODE>(const PartsConfig&, bool, const StepCtx<R>&, const PartsView&, int, \
-                                             cudaStream_t);
+  template const void* parts_fn<R, MODE>(int, bool);                                                            \
+  template cudaError_t launch_parts<R, MODE>(const PartsConfig&, const StepCtx<R>&, const PartsView&, int, cudaStream_t);
 VBD_PARTS(float, MODE_FP32)
 VBD_PARTS(float, MODE_MIXED)
 VBD_PARTS(double, MODE_FP64)

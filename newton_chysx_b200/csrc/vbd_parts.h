@@ -14,7 +14,7 @@ struct PartsView {
   int C;                      // colors
   int P;                      // parts per job
   int njobs;
-  int face_damping;           // some triangle is damped
+  const int* damping;         // kFaceDamping | kHingeDamping: elements with damping (a refresh rewrites it)
   int places, most_own;       // most places and most own particles of a part: the shared-memory layout
   const int* job_order;       // [njobs] largest first
   const int* part_base;       // [parts + 1] own particles of all parts before
@@ -30,11 +30,15 @@ struct PartsView {
   const uint4* faceA;         // the records of vbd_ell.cuh's compact layout with part-local 16-bit places, round
   const uint4* faceB;         //   major: base + (round * n + vertex) * L + lane
   const uint4* hinge;
-  const float* hinge_kd;      // NULL without hinge damping
+  const float* hinge_kd;      // read with kHingeDamping only
   float4* contact;            // [3 V] by place: a particle's only contact with a static shape, as part_contact_add reads it
   int* queue;                 // work counter, zero before launch
   unsigned* done;             // [P * kDoneStride] colors finished by each CTA over its jobs, zero before launch (grid)
 };
+
+// Bits of PartsView::damping. In device memory, as the records are: a captured step follows a refresh that brings
+// damping or takes it away.
+constexpr int kFaceDamping = 1, kHingeDamping = 2;
 
 constexpr int kDoneStride = 32;  // one flag per 128-byte line
 
@@ -51,11 +55,10 @@ struct PartsConfig {
 };
 
 template <typename R, int MODE>
-const void* parts_fn(int L, bool wide, bool damped);
+const void* parts_fn(int L, bool wide);
 
 template <typename R, int MODE>
-cudaError_t launch_parts(const PartsConfig& g, bool damped, const StepCtx<R>& c, const PartsView& p, int iterations,
-                         cudaStream_t st);
+cudaError_t launch_parts(const PartsConfig& g, const StepCtx<R>& c, const PartsView& p, int iterations, cudaStream_t st);
 
 }  // namespace vbd
 
@@ -80,8 +83,8 @@ struct PartsPlan {
 // Cuts the jobs (job_v0: first particle of each job, then V) into P parts each. False: the plan does not exist
 // (a part with 65,536 places or more, or an element with two vertices of one color).
 bool parts_plan(const PartsInput& in, const std::vector<int>& job_v0, int P, int L, PartsPlan& plan);
-// The records of the plan's elements with the input's materials; kd stays empty when no hinge is damped.
-void parts_records(const PartsInput& in, const PartsPlan& plan, bool hinge_damping, std::vector<uint4>& faceA,
+// The records of the plan's elements with the input's materials.
+void parts_records(const PartsInput& in, const PartsPlan& plan, std::vector<uint4>& faceA,
                    std::vector<uint4>& faceB, std::vector<uint4>& hinge, std::vector<float>& kd);
 
 }  // namespace vbd

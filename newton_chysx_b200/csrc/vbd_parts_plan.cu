@@ -156,13 +156,13 @@ bool parts_plan(const PartsInput& in, const std::vector<int>& job_v0, int P, int
   return plan.most_places < 65536;
 }
 
-void parts_records(const PartsInput& in, const PartsPlan& plan, bool hinge_damping, std::vector<uint4>& faceA,
+void parts_records(const PartsInput& in, const PartsPlan& plan, std::vector<uint4>& faceA,
                    std::vector<uint4>& faceB, std::vector<uint4>& hinge, std::vector<float>& kd) {
   const uint4 none = make_uint4(0u, 0u, 0u, 0u);
   faceA.assign(size_t(std::max(plan.faces, 1LL)), none);
   faceB.assign(faceA.size(), none);
   hinge.assign(size_t(std::max(plan.hinges, 1LL)), none);
-  kd.assign(hinge_damping ? hinge.size() : 0, 0.f);
+  kd.assign(hinge.size(), 0.f);
   const int C = plan.C, L = plan.L;
   for_parts(plan.njobs * plan.P, in.V, [&](int part, std::vector<int>& place) {
     const int k0 = plan.part_base[part], k1 = plan.part_base[part + 1];
@@ -203,7 +203,7 @@ void parts_records(const PartsInput& in, const PartsPlan& plan, bool hinge_dampi
         const size_t i = size_t(plan.ebase[r] + ((s / L) * n + j) * L + s % L);
         hinge[i] = make_uint4(unsigned(place[ei[0]]) | (unsigned(place[ei[1]]) << 16),
                               unsigned(place[ei[2]]) | (unsigned(place[ei[3]]) << 16), bits(in.rest_angle[e]), bits(kl));
-        if (hinge_damping) kd[i] = in.bending[2 * size_t(e) + 1];
+        kd[i] = in.bending[2 * size_t(e) + 1];
       }
     }
   });

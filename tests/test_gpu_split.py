@@ -108,11 +108,20 @@ def test_split_worlds_match_the_one_cta_kernel(sides):
     assert np.abs(got - ref).max() <= 1e-4
 
 
+def _damp(model, faces, hinges):
+    model.tri_materials[:, 2] = faces
+    model.edge_bending_properties[:, 1] = hinges
+
+
+# the damping (membranes, hinges) at the capture and after the refresh; 20 x 20 is one cluster, 64 x 64 a grid
 @pytest.mark.parametrize("n", [20, 64])
-def test_split_refresh_and_capture(n):
-    """A graph captured before a refresh steps with the new materials, hinge damping still off, and agrees with an
-    eager step bit for bit; a state stepped in place keeps working."""
+@pytest.mark.parametrize("before,after", [((0.0, 0.0), (0.0, 0.0)), ((0.0, 0.0), (0.0, 2e-3)), ((0.0, 2e-3), (0.0, 0.0)),
+                                          ((0.0, 0.0), (2e-3, 0.0)), ((2e-3, 2e-3), (0.0, 0.0))])  # fmt: skip
+def test_split_refresh_and_capture(n, before, after):
+    """A graph captured before a refresh steps with the new materials, damping that came or went among them, and agrees
+    bit for bit with an eager step and with a new solver; a state stepped in place keeps working."""
     model = _sheet(n, n).finalize("cuda:0")
+    _damp(model, *before)
     q, qd = _start(model, n)
     solver = SolverVBD(model, iterations=5)
     pipe = CollisionPipeline(model, soft_contact_margin=0.01)
@@ -133,18 +142,25 @@ def test_split_refresh_and_capture(n):
         pipe.collide(s0, contacts)
         solver.step(s0, s1, None, contacts, DT)
     torch.cuda.synchronize()
-    model.tri_materials[:, :2] *= 3.0
+    reset()
+    graph.replay()
+    torch.cuda.synchronize()
+    old = s1.particle_q.clone()
+    model.tri_materials[:, :2] *= 3.0 if before == after else 1.0
+    _damp(model, *after)
     solver.notify_model_changed()
     reset()
     graph.replay()
     torch.cuda.synchronize()
     captured = s1.particle_q.clone()
+    assert not torch.equal(captured, old)
     reset()
     pipe.collide(s0, contacts)
     solver.step(s0, s1, None, contacts, DT)
     torch.cuda.synchronize()
     assert torch.equal(captured, s1.particle_q)
     fresh = SolverVBD(model, iterations=5)
+    assert solver.split is not None and fresh.split == solver.split
     reset()
     pipe.collide(s0, contacts)
     fresh.step(s0, s0, None, contacts, DT)
