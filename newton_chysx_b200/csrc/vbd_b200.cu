@@ -236,8 +236,9 @@ struct VbdSolver {
   PartsView pt = {};
   char* pt_blob = nullptr;
   uint4 *pt_faceA = nullptr, *pt_faceB = nullptr, *pt_hinge = nullptr;
-  float* pt_kd = nullptr;
-  int* pt_damping = nullptr;
+  float *pt_area = nullptr, *pt_kd = nullptr;
+  int2* pt_place_of = nullptr;
+  int* pt_flags = nullptr;
   float4* pt_contact = nullptr;
   // adjoint work buffers (allocated by the first vbd_adjoint_step)
   void* adj_work = nullptr;
@@ -263,7 +264,7 @@ struct VbdSolver {
                   ell16_faceA, ell16_faceB, ell16_hinge, sc_pos_cd, sc_disp, sc_ts, ring_nslot, ring_base,
                   ring_vbase, ring_A, ring_B, ring_H, ring_hdr, ring_kd, spr_idx, spr_prop, spr_off, spr_adj, sspr_off,
                   sspr_adj, spr_acc, tet_idx, tet_pose, tet_off, tet_adj, sc_estart, sc_world, pt_blob, color_of_dev, live, pt_faceA, pt_faceB, pt_hinge,
-                  pt_kd, pt_damping, pt_contact};
+                  pt_area, pt_kd, pt_place_of, pt_flags, pt_contact};
     for (void* p : ps)
       if (p) cudaFree(p);
     sc_release(sc);
@@ -671,53 +672,14 @@ int allow_shared(const void* fn) {
   return VBD_OK;
 }
 
-// The records of the split-instance plan from the model's current materials, into the buffers that are there when
-// their sizes are the same (a captured graph keeps reading them).
-template <typename T>
-int upload_same(T** d, const std::vector<T>& h, bool have) {
-  if (!have || !*d) return upload_into(d, h);
-  return h.empty() || cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice) == cudaSuccess
-             ? VBD_OK
-             : VBD_ERR_CUDA;
-}
-
-int parts_input(VbdSolver* h, PartsInput& in, std::vector<float> buf[6]) {
-  const VbdModelDesc& m = h->md;
-  int rc;
-  if ((rc = download(buf[0], m.tri_poses_dev, size_t(4) * h->T)) ||
-      (rc = download(buf[1], m.tri_materials_dev, size_t(5) * h->T)) ||
-      (rc = download(buf[2], m.tri_areas_dev, size_t(h->T))) ||
-      (rc = download(buf[3], m.edge_rest_angle_dev, size_t(h->E))) ||
-      (rc = download(buf[4], m.edge_rest_length_dev, size_t(h->E))) ||
-      (rc = download(buf[5], m.edge_bending_properties_dev, size_t(2) * h->E)))
-    return rc;
+PartsInput parts_input(const VbdSolver* h) {
+  PartsInput in;
   in.V = h->V, in.T = h->T, in.E = h->E;
   in.C = int(h->color_offsets.size()) - 1;
   in.tri = h->h_tri.data(), in.edges = h->h_edges.data();
   in.foff = h->h_foff.data(), in.fadj = h->h_fadj.data(), in.eoff = h->h_eoff.data(), in.eadj = h->h_eadj.data();
   in.color_of = h->color_of.data();
-  in.pose = buf[0].data(), in.mat = buf[1].data(), in.area = buf[2].data();
-  in.rest_angle = buf[3].data(), in.rest_length = buf[4].data(), in.bending = buf[5].data();
-  return VBD_OK;
-}
-
-int upload_parts_records(VbdSolver* h, const PartsInput& in, bool have) {
-  std::vector<int> damping = {0};
-  for (int e = 0; e < h->E; ++e)
-    if (in.bending[2 * size_t(e)] > 0.f && in.bending[2 * size_t(e) + 1] > 0.f) damping[0] |= kHingeDamping;
-  for (int t = 0; t < h->T; ++t) {
-    const float* m = in.mat + 5 * size_t(t);
-    if ((m[0] > 0.f || m[1] > 0.f) && m[2] > 0.f) damping[0] |= kFaceDamping;
-  }
-  std::vector<uint4> fa, fb, hg;
-  std::vector<float> kd;
-  parts_records(in, h->plan, fa, fb, hg, kd);
-  int rc;
-  if ((rc = upload_same(&h->pt_faceA, fa, have)) || (rc = upload_same(&h->pt_faceB, fb, have)) ||
-      (rc = upload_same(&h->pt_hinge, hg, have)) || (rc = upload_same(&h->pt_kd, kd, have)) ||
-      (rc = upload_same(&h->pt_damping, damping, have)))
-    return rc;
-  return VBD_OK;
+  return in;
 }
 
 // The plan's arrays in one allocation and one copy.
@@ -740,16 +702,28 @@ int upload_plan(VbdSolver* h) {
   const int rc = upload(&h->pt_blob, blob);
   if (rc) return rc;
   for (auto& a : at) *a.first = h->pt_blob + a.second;
+  d.C = p.C, d.P = p.P, d.njobs = p.njobs, d.places = p.most_places, d.most_own = p.most_own;
+  return VBD_OK;
+}
+
+PartsModel parts_model(const VbdSolver* h) {
+  return {h->tri_idx, h->tri_pose, h->tri_mat, h->edge_idx, h->edge_prop, h->face_off, h->face_adj, h->edge_off,
+          h->edge_adj, h->color_of_dev, h->pt_place_of};
+}
+
+// The records of the split-instance plan from the packed model, behind pack_model on the same stream.
+int pack_parts(VbdSolver* h, cudaStream_t st) {
+  CK(parts_pack(parts_model(h), h->pt, h->plan.L,
+                {h->pt_faceA, h->pt_faceB, h->pt_hinge, h->pt_area, h->pt_kd, h->pt_flags}, st));
   return VBD_OK;
 }
 
 PartsView parts_view(const VbdSolver* h) {
   PartsView p = h->pt;  // the plan's arrays
-  p.C = h->plan.C, p.P = h->plan.P, p.njobs = h->plan.njobs;
-  p.places = h->plan.most_places, p.most_own = h->plan.most_own;
   p.faceA = h->pt_faceA, p.faceB = h->pt_faceB, p.hinge = h->pt_hinge;
+  p.face_area = h->pt_area;
   p.hinge_kd = h->pt_kd;
-  p.damping = h->pt_damping;
+  p.flags = h->pt_flags;
   p.contact = h->pt_contact;
   p.queue = h->queue;
   p.done = reinterpret_cast<unsigned*>(h->queue + kDoneStride);
@@ -814,11 +788,8 @@ int build_parts(VbdSolver* h, const std::vector<int>& wstart) {
   g.block = std::min(most, std::max(64, (per_color * g.L + 31) / 32 * 32));
   g.wide = !f64 && g.L <= 2 && g.block > narrow;
   if (!g.wide) g.block = std::min(g.block, narrow);
-  std::vector<float> buf[6];
-  PartsInput in;
-  int rc = parts_input(h, in, buf);
-  if (rc) return rc;
-  if (!parts_plan(in, job_v0, g.P, g.L, h->plan)) return VBD_OK;
+  int rc;
+  if (!parts_plan(parts_input(h), job_v0, g.P, g.L, h->plan)) return VBD_OK;
   g.smem = place * size_t(h->plan.most_places) + (place + sizeof(int)) * size_t(h->plan.most_own);
   if (g.smem + 2048 > size_t(optin)) return VBD_OK;
   h->parts = g;
@@ -844,9 +815,21 @@ int build_parts(VbdSolver* h, const std::vector<int>& wstart) {
   }
   if (fit < 1) return VBD_OK;
   h->parts.blocks = g.P * (g.grid ? 1 : std::min(fit, h->plan.njobs));
+  const size_t nf = size_t(std::max(h->plan.faces, 1LL)), ne = size_t(std::max(h->plan.hinges, 1LL));
   if ((rc = upload_plan(h)) || (h->S > 0 && (rc = dalloc(&h->pt_contact, 3 * size_t(V)))) ||
-      (rc = upload_parts_records(h, in, false)))
+      (rc = dalloc(&h->pt_place_of, size_t(V))) || (rc = dalloc(&h->pt_faceA, nf)) || (rc = dalloc(&h->pt_faceB, nf)) ||
+      (rc = dalloc(&h->pt_area, nf)) || (rc = dalloc(&h->pt_hinge, ne)) || (rc = dalloc(&h->pt_kd, ne)) ||
+      (rc = dalloc(&h->pt_flags, 1)))
     return rc;
+  // places of a round that no element fills stay dead
+  CK(cudaMemsetAsync(h->pt_faceA, 0, nf * sizeof(uint4), 0));
+  CK(cudaMemsetAsync(h->pt_faceB, 0, nf * sizeof(uint4), 0));
+  CK(cudaMemsetAsync(h->pt_hinge, 0, ne * sizeof(uint4), 0));
+  CK(cudaMemsetAsync(h->pt_kd, 0, ne * sizeof(float), 0));
+  CK(parts_places(parts_model(h), h->pt, 0));
+  if ((rc = pack_parts(h, 0))) return rc;
+  for (auto* x : {&h->plan.part_of, &h->plan.slot_of, &h->plan.vert, &h->plan.ghost, &h->plan.ghost_part})
+    std::vector<int>().swap(*x);
   h->parts_on = true;
   return VBD_OK;
 }
@@ -2152,8 +2135,14 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
 
 int vbd_refresh_model(VbdHandle h, void* stream) {
   if (!h) return VBD_ERR_INVALID_ARGUMENT;
-  int rc = pack_model(h, (cudaStream_t)stream);
-  if (rc) return rc;
+  int rc;
+  if (h->parts_on && h->layout != VBD_LAYOUT_CSR) {  // materials that the layout refuses without the split, too
+    if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) return VBD_ERR_CUDA;
+    std::vector<float> mat;
+    if ((rc = download(mat, h->md.tri_materials_dev, size_t(5) * h->T))) return rc;
+    if (needs_lnh_floor(mat, h->T)) return VBD_ERR_UNSUPPORTED;
+  }
+  if ((rc = pack_model(h, (cudaStream_t)stream))) return rc;
   if (h->soft) {
     if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) return VBD_ERR_CUDA;
     if ((rc = pack_live(h))) return rc;
@@ -2164,14 +2153,7 @@ int vbd_refresh_model(VbdHandle h, void* stream) {
     for (int e = 0; e < h->E; ++e)
       if (bp[2 * e] > 0.f && bp[2 * e + 1] > 0.f) return VBD_ERR_UNSUPPORTED;
   }
-  if (h->parts_on) {
-    if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) return VBD_ERR_CUDA;
-    std::vector<float> buf[6];
-    PartsInput in;
-    if ((rc = parts_input(h, in, buf))) return rc;
-    if (needs_lnh_floor(buf[1], h->T)) return VBD_ERR_UNSUPPORTED;
-    return upload_parts_records(h, in, true);
-  }
+  if (h->parts_on) return h->sc_on ? VBD_OK : pack_parts(h, (cudaStream_t)stream);
   if (h->layout == VBD_LAYOUT_ELL || h->layout == VBD_LAYOUT_ELL16 || h->layout == VBD_LAYOUT_RING) {
     if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) return VBD_ERR_CUDA;
     if (h->layout == VBD_LAYOUT_RING) {

@@ -137,7 +137,7 @@ __device__ __forceinline__ int lay_contact(const StepCtx<R>& c, const PartsView&
 
 // One vertex by L lanes (all lanes of the warp call this). fb, eb: this lane's first records; stride: records per
 // round.
-template <typename R, int MODE, int L, bool HD, bool EARLY>
+template <typename R, int MODE, int L, bool GENERAL, bool EARLY>
 __device__ __forceinline__ void solve_part(const StepCtx<R>& c, const PartsView& p, pos4_t<R>* s_pos,
                                            const pos4_t<R>* s_y, const int* s_kind, const int v0,
                                            const PartStart<R>& start, int slot, bool valid, int lane, int nf, int ne,
@@ -169,7 +169,7 @@ __device__ __forceinline__ void solve_part(const StepCtx<R>& c, const PartsView&
     const uint4* pa = p.faceA + fb;
     const uint4* pb = p.faceB + fb;
     const uint4* ph = p.hinge + eb;
-    const float* pk = HD ? p.hinge_kd + eb : nullptr;
+    const float* pk = GENERAL ? p.hinge_kd + eb : nullptr;
     uint4 A_n = make_uint4(0u, 0u, 0u, 0u), B_n = A_n, h_n = A_n;
     if (nf > 0) A_n = __ldg(pa), B_n = __ldg(pb);
     if (ne > 0) h_n = __ldg(ph);  // the first hinge record loads under the faces
@@ -181,20 +181,27 @@ __device__ __forceinline__ void solve_part(const StepCtx<R>& c, const PartsView&
         A_n = __ldg(pa);
         B_n = __ldg(pb);
       }
+      if (!(A.x & kRecordLive)) continue;
       const float muA = __uint_as_float(A.y), lmA = __uint_as_float(A.z);
-      if (!(muA > 0.f || lmA > 0.f)) continue;
       const R pose[4] = {R(__uint_as_float(A.w)), R(__uint_as_float(B.x)), R(__uint_as_float(B.y)),
                          R(__uint_as_float(B.z))};
       const float kd = __uint_as_float(B.w);
-      const int ia = int(A.x & 0xffffu), ib = int(A.x >> 16);
+      const int ia = int(A.x & (kMostPlaces - 1)), ib = int((A.x >> 16) & (kMostPlaces - 1));
       vec3<R> xp[3];
       if (kd > 0.f) xp[0] = start.ld(slot), xp[1] = start.ld(ia), xp[2] = start.ld(ib);
+      if constexpr (GENERAL) {
+        if (A.x & kRecordFloor) {
+          const R lnh_floor = R(1.0e-6) * R(__ldg(p.face_area + fb + (long long)s * stride));
+          membrane_add<R>(0, x, pos.ld(ia), pos.ld(ib), pose, R(muA), R(lmA), R(kd), R(1), c.dt, xp, f, H, lnh_floor);
+          continue;
+        }
+      }
       membrane_add<R>(0, x, pos.ld(ia), pos.ld(ib), pose, R(muA), R(lmA), R(kd), R(1), c.dt, xp, f, H, R(0));
     }
     for (int s = 0; s < ne; ++s) {
       const uint4 hh = h_n;
       float kd = 0.f;
-      if constexpr (HD) {
+      if constexpr (GENERAL) {
         kd = __ldg(pk);
         pk += stride;
       }
@@ -202,9 +209,10 @@ __device__ __forceinline__ void solve_part(const StepCtx<R>& c, const PartsView&
         ph += stride;
         h_n = __ldg(ph);
       }
+      if (!(hh.y & kRecordLive)) continue;
       const float k = __uint_as_float(hh.w);
-      if (!(k > 0.f)) continue;
-      const int i0 = int(hh.x & 0xffffu), i1 = int(hh.x >> 16), i2 = int(hh.y & 0xffffu), i3 = int(hh.y >> 16);
+      const int i0 = int(hh.x & 0xffffu), i1 = int(hh.x >> 16);
+      const int i2 = int(hh.y & 0xffffu), i3 = int((hh.y >> 16) & (kMostPlaces - 1));
       // the solved vertex's role is where its place appears (bending_add_coef's constants)
       const bool r0 = i0 == slot, r1 = i1 == slot, r2 = i2 == slot, r3 = !(r0 || r1 || r2);
       const R ca = r0 ? R(-1) : (r2 ? R(1) : R(0));
@@ -212,7 +220,7 @@ __device__ __forceinline__ void solve_part(const StepCtx<R>& c, const PartsView&
       const R dd = r2 ? R(1) : (r3 ? R(-1) : R(0));
       const vec3<R> xs[4] = {pos.ld(i0), pos.ld(i1), pos.ld(i2), pos.ld(i3)};
       const R rest = R(__uint_as_float(hh.z));
-      if constexpr (HD) {
+      if constexpr (GENERAL) {
         if (kd > 0.f) {
           const vec3<R> xp[4] = {start.ld(i0), start.ld(i1), start.ld(i2), start.ld(i3)};
           bending_add_coef<R>(ca, cb, dd, xs, rest, R(1), R(k), R(kd), c.dt, xp, f, H);
@@ -290,7 +298,7 @@ struct PartShared {
 };
 
 // The iterations of one job. False: a wait ran out.
-template <typename R, int MODE, int L, bool HD, bool EARLY>
+template <typename R, int MODE, int L, bool GENERAL, bool EARLY>
 __device__ __forceinline__ bool sweep_part(const StepCtx<R>& c, const PartsView& p, PartShared& s, pos4_t<R>* s_pos,
                                            const pos4_t<R>* s_y, const int* s_kind, int v0, int nown, int g0,
                                            const PartStart<R>& start, int rank, int grid_mode, int iterations,
@@ -308,7 +316,7 @@ __device__ __forceinline__ bool sweep_part(const StepCtx<R>& c, const PartsView&
       for (int base = 0; base < n; base += per_round) {
         const int j = base + group;
         const long long o = (long long)j * L + lane;
-        solve_part<R, MODE, L, HD, EARLY>(c, p, s_pos, s_y, s_kind, v0, start, a + j, j < n, lane, nf, ne,
+        solve_part<R, MODE, L, GENERAL, EARLY>(c, p, s_pos, s_y, s_kind, v0, start, a + j, j < n, lane, nf, ne,
                                                      fb + o, eb + o, n * L, it);
       }
       if (p.P > 1) {
@@ -347,7 +355,7 @@ __global__ void __launch_bounds__(T, 1)
   namespace cg = cooperative_groups;
   const int rank = grid_mode ? int(blockIdx.x) : int(cg::this_cluster().block_rank());
   const int tid = threadIdx.x, nt = blockDim.x;
-  const int damping = *p.damping;
+  const int flags = *p.flags;
   unsigned phase = 0;
   if (tid == 0) s.abort = 0;
   for (int round = 0;; ++round) {
@@ -401,17 +409,18 @@ __global__ void __launch_bounds__(T, 1)
         s_pos[nown + g - g0] = pk4(predict(c, __ldg(p.ghost + g), q, ms), R(0));
       }
     __syncthreads();
-    // one sweep for each answer to whether hinges are damped: deciding per hinge took 5 % (32 x 32, 256 x 256) to 13 %
-    // (512 worlds) of an undamped step, this 1 (512 x 512) to 3 % (32 x 32: 4 us) against a kernel of its own for each,
-    // between which a captured step could not change
-    const bool done = damping & kHingeDamping
+    // A sweep of its own for models without damped hinges and triangles under the floor: deciding per element took 5 %
+    // (32 x 32, 256 x 256) to 13 % (512 worlds) of their steps for the hinges and 3 to 8 % for the floor. Both in one
+    // kernel take 1 (512 x 512) to 3 % (32 x 32: 4 us) against two kernels, between which a captured step could not
+    // change.
+    const bool done = flags & (kHingeDamping | kFloor)
                           ? sweep_part<R, MODE, L, true, (T <= 512)>(c, p, s, s_pos, s_y, s_kind, v0, nown, g0, start,
                                                                      rank, grid_mode, iterations, phase)
                           : sweep_part<R, MODE, L, false, (T <= 512)>(c, p, s, s_pos, s_y, s_kind, v0, nown, g0, start,
                                                                       rank, grid_mode, iterations, phase);
     if (!done) return;
     // the damping terms read ghosts' start positions from state_in: their owners write it back when all have finished
-    if (grid_mode && damping) {
+    if (grid_mode && (flags & (kFaceDamping | kHingeDamping))) {
       for (int g = g0 + tid; g < g1; g += nt)
         if (!wait_done(p.done + __ldg(p.ghost_part + g) * kDoneStride, phase)) s.abort = 1;
       __syncthreads();

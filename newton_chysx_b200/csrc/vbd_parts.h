@@ -14,7 +14,7 @@ struct PartsView {
   int C;                      // colors
   int P;                      // parts per job
   int njobs;
-  const int* damping;         // kFaceDamping | kHingeDamping: elements with damping (a refresh rewrites it)
+  const int* flags;           // kFaceDamping, kHingeDamping, kFloor (a refresh rewrites it)
   int places, most_own;       // most places and most own particles of a part: the shared-memory layout
   const int* job_order;       // [njobs] largest first
   const int* part_base;       // [parts + 1] own particles of all parts before
@@ -27,18 +27,24 @@ struct PartsView {
   const int* ne;              // [parts, C] hinge rounds
   const long long* fbase;     // [parts, C] first face record
   const long long* ebase;
-  const uint4* faceA;         // the records of vbd_ell.cuh's compact layout with part-local 16-bit places, round
-  const uint4* faceB;         //   major: base + (round * n + vertex) * L + lane
-  const uint4* hinge;
-  const float* hinge_kd;      // read with kHingeDamping only
+  const uint4* faceA;         // the records of vbd_ell.cuh's compact layout with part-local 14-bit places (at bits 0 and
+  const uint4* faceB;         //   16 of a word) and kRecordLive, round major: base + (round * n + vertex) * L + lane
+  const uint4* hinge;         // places in words 0 and 1, kRecordLive in word 1
+  const float* face_area;     // read for records with kRecordFloor
+  const float* hinge_kd;      // read with kHingeDamping or kFloor
   float4* contact;            // [3 V] by place: a particle's only contact with a static shape, as part_contact_add reads it
   int* queue;                 // work counter, zero before launch
   unsigned* done;             // [P * kDoneStride] colors finished by each CTA over its jobs, zero before launch (grid)
 };
 
-// Bits of PartsView::damping. In device memory, as the records are: a captured step follows a refresh that brings
-// damping or takes it away.
-constexpr int kFaceDamping = 1, kHingeDamping = 2;
+constexpr int kMostPlaces = 1 << 14;  // the shared memory of an SM holds fewer
+// Flags of a record's word beside its places. Live: the element has stiffness. Floor: |lambda + mu| is under the reference's
+// floor of 1e-6, which the kernel applies to the coefficients times the area.
+constexpr unsigned kRecordLive = 1u << 31, kRecordFloor = 1u << 30;
+
+// Bits of PartsView::flags: some triangle, some hinge is damped, some record has kRecordFloor. In device memory, as the
+// records are: a captured step follows a refresh that brings one of them or takes it away.
+constexpr int kFaceDamping = 1, kHingeDamping = 2, kFloor = 4;
 
 constexpr int kDoneStride = 32;  // one flag per 128-byte line
 
@@ -64,14 +70,12 @@ cudaError_t launch_parts(const PartsConfig& g, const StepCtx<R>& c, const PartsV
 
 namespace vbd {
 
-// The host side of a plan: the cut, the places, the ghosts and the record layout (topology only), and the records.
+// The host side of a plan: the cut, the places, the ghosts and the layout of the records (topology only).
 struct PartsInput {
   int V = 0, T = 0, E = 0, C = 0;
-  const int *tri = nullptr, *edges = nullptr;                                             // topology
-  const int *foff = nullptr, *fadj = nullptr, *eoff = nullptr, *eadj = nullptr;           // packed adjacency
-  const int* color_of = nullptr;                                                          // [V]
-  const float *pose = nullptr, *mat = nullptr, *area = nullptr;                           // triangles
-  const float *rest_angle = nullptr, *rest_length = nullptr, *bending = nullptr;          // hinges
+  const int *tri = nullptr, *edges = nullptr;                                    // topology
+  const int *foff = nullptr, *fadj = nullptr, *eoff = nullptr, *eadj = nullptr;  // packed adjacency
+  const int* color_of = nullptr;                                                 // [V]
 };
 struct PartsPlan {
   int P = 0, L = 1, njobs = 0, C = 0, most_places = 0, most_own = 0;
@@ -81,10 +85,26 @@ struct PartsPlan {
 };
 
 // Cuts the jobs (job_v0: first particle of each job, then V) into P parts each. False: the plan does not exist
-// (a part with 65,536 places or more, or an element with two vertices of one color).
+// (a part with kMostPlaces places or more, or an element with two vertices of one color).
 bool parts_plan(const PartsInput& in, const std::vector<int>& job_v0, int P, int L, PartsPlan& plan);
-// The records of the plan's elements with the input's materials.
-void parts_records(const PartsInput& in, const PartsPlan& plan, std::vector<uint4>& faceA,
-                   std::vector<uint4>& faceB, std::vector<uint4>& hinge, std::vector<float>& kd);
+
+// The records from the packed model (device arrays of StepCtx), written by kernels on `st` where they stand, so that a
+// refresh needs no synchronisation and captured steps read the new ones.
+struct PartsModel {
+  const int4* tri_idx;
+  const float4 *tri_pose, *tri_mat;
+  const int4* edge_idx;
+  const float4* edge_prop;
+  const int *face_off, *face_adj, *edge_off, *edge_adj;
+  const int* color_of;
+  int2* place_of;  // [V] part and own place of each particle
+};
+struct PartsRecords {
+  uint4 *faceA, *faceB, *hinge;
+  float *face_area, *hinge_kd;
+  int* flags;
+};
+cudaError_t parts_places(const PartsModel& m, const PartsView& p, cudaStream_t st);  // place_of, once per plan
+cudaError_t parts_pack(const PartsModel& m, const PartsView& p, int L, const PartsRecords& r, cudaStream_t st);
 
 }  // namespace vbd

@@ -14,7 +14,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 import newton_chysx_b200 as nb  # noqa: E402
-from newton_chysx_b200 import CollisionPipeline, SolverVBD  # noqa: E402
+from newton_chysx_b200 import CollisionPipeline, SolverVBD, _lib  # noqa: E402
 from tests.helpers import cloth_grid_builder  # noqa: E402
 
 DT = 1.0 / 600.0
@@ -167,6 +167,74 @@ def test_split_refresh_and_capture(n, before, after):
     torch.cuda.synchronize()
     assert torch.equal(captured, s0.particle_q)
     del graph
+
+
+@pytest.mark.parametrize("n", [20, 41])
+def test_split_refresh_inside_a_capture(n):
+    """A refresh of a default cloth launches kernels only: captured with the step, a replay takes the materials that the
+    model holds by then. The same kernels on the same data as an eager refresh and step: bit for bit."""
+    model = _sheet(n, n).finalize("cuda:0")
+    q, qd = (torch.as_tensor(x, device="cuda") for x in _start(model, n))
+    solver = SolverVBD(model, iterations=5)
+    assert solver.split is not None and solver.layout == "csr"
+    s0, s1 = model.state(), model.state()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream):
+        s0.particle_q.copy_(q)
+        s0.particle_qd.copy_(qd)
+        solver.notify_model_changed()
+        solver.step(s0, s1, None, None, DT)
+    out = []
+    for scale, hinges in ((1.0, 0.0), (3.0, 2e-3)):
+        model.tri_materials[:, :2] *= scale
+        _damp(model, 0.0, hinges)
+        graph.replay()
+        torch.cuda.synchronize()
+        out.append(s1.particle_q.clone())
+        s0.particle_q.copy_(q)
+        s0.particle_qd.copy_(qd)
+        SolverVBD(model, iterations=5).step(s0, s1, None, None, DT)
+        torch.cuda.synchronize()
+        assert torch.equal(out[-1], s1.particle_q)
+    assert not torch.equal(*out)
+    del graph
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_split_refresh_takes_materials_under_the_floor(precision):
+    """A refresh to triangles with |lambda + mu| < 1e-6 needs the reference's floor on the material values: a default cloth
+    takes it, as its csr layout does unsplit; a named ell16 layout refuses it and keeps the materials it had."""
+    model = _sheet(24, 24).finalize("cuda:0")
+    q, qd = (torch.as_tensor(x, device="cuda") for x in _start(model, 3))
+    solvers = [SolverVBD(model, iterations=5, precision=precision, **kw)
+               for kw in ({}, dict(layout="csr", schedule="persistent", lanes_per_vertex=1), dict(layout="ell16", schedule="persistent"))]  # fmt: skip
+    assert [s.split is not None for s in solvers] == [True, False, True]
+
+    def step(solver):
+        a, b = model.state(), model.state()
+        if precision == "fp64":
+            for s in (a, b):
+                s.particle_f = None
+                s.particle_q, s.particle_qd = s.particle_q.double(), s.particle_qd.double()
+        a.particle_q.copy_(q)
+        a.particle_qd.copy_(qd)
+        solver.step(a, b, None, None, DT)
+        torch.cuda.synchronize()
+        assert solver.device_errors() == 0
+        return b.particle_q.double()
+
+    before = step(solvers[2])
+    model.tri_materials[::3, 0], model.tri_materials[::3, 1] = 4.0e-7, 1.0e-7
+    model.tri_materials[1::7, 0], model.tri_materials[1::7, 1] = 2.0, -2.0
+    for solver in solvers[:2]:
+        solver.notify_model_changed()
+    with pytest.raises(_lib.VbdError, match="unsupported"):
+        solvers[2].notify_model_changed()
+    assert torch.equal(step(solvers[2]), before)
+    got, ref = step(solvers[0]), step(solvers[1])
+    assert not torch.equal(got, before)
+    assert (got - ref).abs().max().item() <= (1e-9 if precision == "fp64" else 1e-5)
 
 
 def test_what_steps_split_and_what_does_not():
