@@ -236,7 +236,7 @@ struct VbdSolver {
   PartsView pt = {};
   char* pt_blob = nullptr;
   uint4 *pt_faceA = nullptr, *pt_faceB = nullptr, *pt_hinge = nullptr;
-  float *pt_area = nullptr, *pt_kd = nullptr;
+  float *pt_area = nullptr, *pt_length = nullptr, *pt_kd = nullptr;
   int2* pt_place_of = nullptr;
   int* pt_flags = nullptr;
   float4* pt_contact = nullptr;
@@ -264,7 +264,7 @@ struct VbdSolver {
                   ell16_faceA, ell16_faceB, ell16_hinge, sc_pos_cd, sc_disp, sc_ts, ring_nslot, ring_base,
                   ring_vbase, ring_A, ring_B, ring_H, ring_hdr, ring_kd, spr_idx, spr_prop, spr_off, spr_adj, sspr_off,
                   sspr_adj, spr_acc, tet_idx, tet_pose, tet_off, tet_adj, sc_estart, sc_world, pt_blob, color_of_dev, live, pt_faceA, pt_faceB, pt_hinge,
-                  pt_area, pt_kd, pt_place_of, pt_flags, pt_contact};
+                  pt_area, pt_length, pt_kd, pt_place_of, pt_flags, pt_contact};
     for (void* p : ps)
       if (p) cudaFree(p);
     sc_release(sc);
@@ -713,8 +713,8 @@ PartsModel parts_model(const VbdSolver* h) {
 
 // The records of the split-instance plan from the packed model, behind pack_model on the same stream.
 int pack_parts(VbdSolver* h, cudaStream_t st) {
-  CK(parts_pack(parts_model(h), h->pt, h->plan.L,
-                {h->pt_faceA, h->pt_faceB, h->pt_hinge, h->pt_area, h->pt_kd, h->pt_flags}, st));
+  CK(parts_pack(parts_model(h), h->pt, h->plan.L, h->precision == VBD_PRECISION_FP64,
+                {h->pt_faceA, h->pt_faceB, h->pt_hinge, h->pt_area, h->pt_length, h->pt_kd, h->pt_flags}, st));
   return VBD_OK;
 }
 
@@ -722,6 +722,7 @@ PartsView parts_view(const VbdSolver* h) {
   PartsView p = h->pt;  // the plan's arrays
   p.faceA = h->pt_faceA, p.faceB = h->pt_faceB, p.hinge = h->pt_hinge;
   p.face_area = h->pt_area;
+  p.hinge_length = h->pt_length;
   p.hinge_kd = h->pt_kd;
   p.flags = h->pt_flags;
   p.contact = h->pt_contact;
@@ -818,7 +819,8 @@ int build_parts(VbdSolver* h, const std::vector<int>& wstart) {
   const size_t nf = size_t(std::max(h->plan.faces, 1LL)), ne = size_t(std::max(h->plan.hinges, 1LL));
   if ((rc = upload_plan(h)) || (h->S > 0 && (rc = dalloc(&h->pt_contact, 3 * size_t(V)))) ||
       (rc = dalloc(&h->pt_place_of, size_t(V))) || (rc = dalloc(&h->pt_faceA, nf)) || (rc = dalloc(&h->pt_faceB, nf)) ||
-      (rc = dalloc(&h->pt_area, nf)) || (rc = dalloc(&h->pt_hinge, ne)) || (rc = dalloc(&h->pt_kd, ne)) ||
+      (rc = dalloc(&h->pt_area, nf)) || (rc = dalloc(&h->pt_hinge, ne)) || (rc = dalloc(&h->pt_length, ne)) ||
+      (rc = dalloc(&h->pt_kd, ne)) ||
       (rc = dalloc(&h->pt_flags, 1)))
     return rc;
   // places of a round that no element fills stay dead

@@ -188,6 +188,15 @@ __device__ __forceinline__ void solve_part(const StepCtx<R>& c, const PartsView&
       const float kd = __uint_as_float(B.w);
       const int ia = int(A.x & (kMostPlaces - 1)), ib = int((A.x >> 16) & (kMostPlaces - 1));
       vec3<R> xp[3];
+      if constexpr (sizeof(R) == 8) {
+        const int ord = int((A.x >> 14) & 3u);  // the triangle's vertices in its own order: (slot, a, b) from vertex `ord` on
+        const int i0 = ord == 0 ? slot : (ord == 1 ? ib : ia), i1 = ord == 0 ? ia : (ord == 1 ? slot : ib);
+        const int i2 = ord == 0 ? ib : (ord == 1 ? ia : slot);
+        if (kd > 0.f) xp[0] = start.ld(i0), xp[1] = start.ld(i1), xp[2] = start.ld(i2);
+        const R area = R(__ldg(p.face_area + fb + (long long)s * stride));
+        membrane_add<R>(ord, pos.ld(i0), pos.ld(i1), pos.ld(i2), pose, R(muA), R(lmA), R(kd), area, c.dt, xp, f, H);
+        continue;
+      }
       if (kd > 0.f) xp[0] = start.ld(slot), xp[1] = start.ld(ia), xp[2] = start.ld(ib);
       if constexpr (GENERAL) {
         if (A.x & kRecordFloor) {
@@ -211,6 +220,8 @@ __device__ __forceinline__ void solve_part(const StepCtx<R>& c, const PartsView&
       }
       if (!(hh.y & kRecordLive)) continue;
       const float k = __uint_as_float(hh.w);
+      R length = R(1);
+      if constexpr (sizeof(R) == 8) length = R(__ldg(p.hinge_length + eb + (long long)s * stride));
       const int i0 = int(hh.x & 0xffffu), i1 = int(hh.x >> 16);
       const int i2 = int(hh.y & 0xffffu), i3 = int((hh.y >> 16) & (kMostPlaces - 1));
       // the solved vertex's role is where its place appears (bending_add_coef's constants)
@@ -223,11 +234,11 @@ __device__ __forceinline__ void solve_part(const StepCtx<R>& c, const PartsView&
       if constexpr (GENERAL) {
         if (kd > 0.f) {
           const vec3<R> xp[4] = {start.ld(i0), start.ld(i1), start.ld(i2), start.ld(i3)};
-          bending_add_coef<R>(ca, cb, dd, xs, rest, R(1), R(k), R(kd), c.dt, xp, f, H);
+          bending_add_coef<R>(ca, cb, dd, xs, rest, length, R(k), R(kd), c.dt, xp, f, H);
           continue;
         }
       }
-      bending_add_coef<R>(ca, cb, dd, xs, rest, R(1), R(k), R(0), c.dt, nullptr, f, H);
+      bending_add_coef<R>(ca, cb, dd, xs, rest, length, R(k), R(0), c.dt, nullptr, f, H);
     }
   }
   if (L > 1) {

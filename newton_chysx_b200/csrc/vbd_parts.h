@@ -30,7 +30,10 @@ struct PartsView {
   const uint4* faceA;         // the records of vbd_ell.cuh's compact layout with part-local 14-bit places (at bits 0 and
   const uint4* faceB;         //   16 of a word) and kRecordLive, round major: base + (round * n + vertex) * L + lane
   const uint4* hinge;         // places in words 0 and 1, kRecordLive in word 1
-  const float* face_area;     // read for records with kRecordFloor
+                              // FP64: as the csr layout reads its elements, the rest inverse of the triangle's own order
+                              //   (the solved vertex's at bit 14 of faceA's places), mu, lambda and ke unscaled
+  const float* face_area;     // read in FP64 and for records with kRecordFloor
+  const float* hinge_length;  // read in FP64
   const float* hinge_kd;      // read with kHingeDamping or kFloor
   float4* contact;            // [3 V] by place: a particle's only contact with a static shape, as part_contact_add reads it
   int* queue;                 // work counter, zero before launch
@@ -101,10 +104,11 @@ struct PartsModel {
 };
 struct PartsRecords {
   uint4 *faceA, *faceB, *hinge;
-  float *face_area, *hinge_kd;
+  float *face_area, *hinge_length, *hinge_kd;
   int* flags;
 };
 cudaError_t parts_places(const PartsModel& m, const PartsView& p, cudaStream_t st);  // place_of, once per plan
-cudaError_t parts_pack(const PartsModel& m, const PartsView& p, int L, const PartsRecords& r, cudaStream_t st);
+cudaError_t parts_pack(const PartsModel& m, const PartsView& p, int L, bool f64, const PartsRecords& r,
+                       cudaStream_t st);
 
 }  // namespace vbd

@@ -159,6 +159,7 @@ __global__ void k_parts_places(const PartsView p, int2* place_of) {
 // A block per part and slice of its particles, a thread per particle. A refresh of 512 worlds of side U{16..128} (3.3 M
 // particles, 1.3 GB of records) replaces 1.1 s of host loops and uploads.
 constexpr int kPackSlices = 4;
+template <bool F64>
 __global__ void __launch_bounds__(256) k_parts_pack(const PartsModel m, const PartsView p, int L, const PartsRecords r) {
   const int part = blockIdx.x, C = p.C;
   const int k0 = p.part_base[part], k1 = p.part_base[part + 1], nown = k1 - k0;
@@ -191,27 +192,34 @@ __global__ void __launch_bounds__(256) k_parts_pack(const PartsModel m, const Pa
       const int4 ti = m.tri_idx[t];
       const float4 D = m.tri_pose[t], mat = m.tri_mat[t];  // mat: mu, lambda, damping, area
       const size_t i = size_t(p.fbase[range] + ((s / L) * n + j) * L + s % L);
+      const double area = mat.w;
       const float mu = mat.x * mat.w, lambda = mat.y * mat.w;
-      if (!(mu > 0.f || lambda > 0.f)) {
+      if (!(F64 ? mat.x * area > 0.0 || mat.y * area > 0.0 : mu > 0.f || lambda > 0.f)) {
         r.faceA[i] = r.faceB[i] = make_uint4(0u, 0u, 0u, 0u);
         continue;
       }
       if (mat.z > 0.f) flags |= kFaceDamping;
+      const unsigned a = place(ord == 0 ? ti.y : (ord == 1 ? ti.z : ti.x));
+      const unsigned b = place(ord == 0 ? ti.z : (ord == 1 ? ti.x : ti.y));
+      r.face_area[i] = mat.w;
+      if constexpr (F64) {  // products and a re-expressed rest inverse rounded to FP32 would cost 1e-12 m per substep
+        r.faceA[i] = make_uint4(a | (unsigned(ord) << 14) | (b << 16) | kRecordLive, __float_as_uint(mat.x),
+                                __float_as_uint(mat.y), __float_as_uint(D.x));
+        r.faceB[i] = make_uint4(__float_as_uint(D.y), __float_as_uint(D.z), __float_as_uint(D.w), __float_as_uint(mat.z));
+        continue;
+      }
       // the solved vertex as vertex 0 of the triangle: the rest inverse re-expressed for that (vbd_ell.cuh)
       double P00 = D.x, P01 = D.y, P10 = D.z, P11 = D.w;
       if (ord == 1)
         P00 = D.z, P01 = D.w, P10 = -double(D.x) - D.z, P11 = -double(D.y) - D.w;
       else if (ord == 2)
         P00 = -double(D.x) - D.z, P01 = -double(D.y) - D.w, P10 = D.x, P11 = D.y;
-      const unsigned a = place(ord == 0 ? ti.y : (ord == 1 ? ti.z : ti.x));
-      const unsigned b = place(ord == 0 ? ti.z : (ord == 1 ? ti.x : ti.y));
       const unsigned floor = fabsf(mat.y + mat.x) >= 1.0e-6f ? 0u : kRecordFloor;
       if (floor) flags |= kFloor;
       r.faceA[i] = make_uint4(a | (b << 16) | kRecordLive | floor, __float_as_uint(mu),
                               __float_as_uint(lambda), __float_as_uint(float(P00)));
       r.faceB[i] = make_uint4(__float_as_uint(float(P01)), __float_as_uint(float(P10)), __float_as_uint(float(P11)),
                               __float_as_uint(mat.z));
-      r.face_area[i] = mat.w;
     }
     s = 0;
     for (int q = m.edge_off[v]; q < m.edge_off[v + 1]; ++q, ++s) {
@@ -226,7 +234,8 @@ __global__ void __launch_bounds__(256) k_parts_pack(const PartsModel m, const Pa
       }
       if (pr.w > 0.f) flags |= kHingeDamping;
       r.hinge[i] = make_uint4(place(ei.x) | (place(ei.y) << 16), place(ei.z) | (place(ei.w) << 16) | kRecordLive,
-                              __float_as_uint(pr.x), __float_as_uint(pr.z * pr.y));
+                              __float_as_uint(pr.x), __float_as_uint(F64 ? pr.z : pr.z * pr.y));
+      r.hinge_length[i] = pr.y;
       r.hinge_kd[i] = pr.w;
     }
   }
@@ -240,10 +249,15 @@ cudaError_t parts_places(const PartsModel& m, const PartsView& p, cudaStream_t s
   return cudaGetLastError();
 }
 
-cudaError_t parts_pack(const PartsModel& m, const PartsView& p, int L, const PartsRecords& r, cudaStream_t st) {
+cudaError_t parts_pack(const PartsModel& m, const PartsView& p, int L, bool f64, const PartsRecords& r,
+                       cudaStream_t st) {
   const cudaError_t rc = cudaMemsetAsync(r.flags, 0, sizeof(int), st);
   if (rc != cudaSuccess) return rc;
-  k_parts_pack<<<dim3(p.njobs * p.P, kPackSlices), 256, 0, st>>>(m, p, L, r);
+  const dim3 grid(p.njobs * p.P, kPackSlices);
+  if (f64)
+    k_parts_pack<true><<<grid, 256, 0, st>>>(m, p, L, r);
+  else
+    k_parts_pack<false><<<grid, 256, 0, st>>>(m, p, L, r);
   return cudaGetLastError();
 }
 
