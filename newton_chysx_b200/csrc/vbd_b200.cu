@@ -61,6 +61,13 @@ __global__ void k_pack_tris(int T, const int* __restrict__ idx, const float* __r
   o_mat[t] = make_float4(mat[5 * t], mat[5 * t + 1], mat[5 * t + 2], area[t]);
 }
 
+// Soft models: whether any triangle, any hinge has stiffness (StepCtx::live, zero before).
+__global__ void k_pack_live(int T, const float4* __restrict__ tri_mat, int E, const float4* __restrict__ edge_prop,
+                            int* live) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < T && (tri_mat[i].x > 0.f || tri_mat[i].y > 0.f)) live[0] = 1;
+  if (i < E && edge_prop[i].z > 0.f) live[1] = 1;
+}
 __global__ void k_pack_edges(int E, const int* __restrict__ idx, const float* __restrict__ ra,
                              const float* __restrict__ rl, const float* __restrict__ bp, int4* o_idx, float4* o_prop) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -865,20 +872,6 @@ EllView ell_view(const VbdSolver* h) {
   return e;
 }
 
-// Soft models: whether any triangle, any hinge has stiffness, for the kernels (StepCtx::live).
-int pack_live(VbdSolver* h) {
-  std::vector<float> tm, bp;
-  int rc;
-  if ((rc = download(tm, h->md.tri_materials_dev, size_t(5) * h->T)) ||
-      (rc = download(bp, h->md.edge_bending_properties_dev, size_t(2) * h->E)))
-    return rc;
-  int live[2] = {0, 0};
-  for (int t = 0; t < h->T; ++t) live[0] |= tm[5 * t] > 0.f || tm[5 * t + 1] > 0.f;
-  for (int e = 0; e < h->E; ++e) live[1] |= bp[2 * e] > 0.f;
-  CK(cudaMemcpy(h->live, live, sizeof(live), cudaMemcpyHostToDevice));
-  return VBD_OK;
-}
-
 int pack_model(VbdSolver* h, cudaStream_t st) {
   const VbdModelDesc& m = h->md;
   if (h->T > 0) {
@@ -901,6 +894,12 @@ int pack_model(VbdSolver* h, cudaStream_t st) {
   if (h->NT > 0) {
     k_pack_tets<<<(h->NT + 255) / 256, 256, 0, st>>>(h->NT, m.tet_indices_dev, m.tet_poses_dev, m.tet_materials_dev,
                                                       h->tet_idx, h->tet_pose);
+    CK(cudaGetLastError());
+  }
+  if (h->soft) {
+    CK(cudaMemsetAsync(h->live, 0, 2 * sizeof(int), st));
+    const int n = std::max(h->T, h->E);
+    if (n > 0) k_pack_live<<<(n + 255) / 256, 256, 0, st>>>(h->T, h->tri_mat, h->E, h->edge_prop, h->live);
     CK(cudaGetLastError());
   }
   return VBD_OK;
@@ -1930,7 +1929,7 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
       return fail(rc);
     if (h->n_same_springs && (rc = dalloc((char**)&h->spr_acc, racc * 9 * size_t(h->V)))) return fail(rc);
   }
-  if ((rc = pack_model(h, 0)) || (soft && (rc = pack_live(h)))) return fail(rc);
+  if ((rc = pack_model(h, 0))) return fail(rc);
 
   // instances (worlds)
   std::vector<int> wstart;
@@ -2145,10 +2144,6 @@ int vbd_refresh_model(VbdHandle h, void* stream) {
     if (needs_lnh_floor(mat, h->T)) return VBD_ERR_UNSUPPORTED;
   }
   if ((rc = pack_model(h, (cudaStream_t)stream))) return rc;
-  if (h->soft) {
-    if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) return VBD_ERR_CUDA;
-    if ((rc = pack_live(h))) return rc;
-  }
   if (h->pair && h->E) {  // the paired kernel has no hinge damping term
     std::vector<float> bp;
     if ((rc = download(bp, h->md.edge_bending_properties_dev, size_t(2) * h->E))) return rc;

@@ -90,3 +90,30 @@ def test_surface_stiffness_comes_and_goes(schedule, same_color_spring):
             bare = got
         else:
             assert float((got - bare).abs().max()) > 1e-9  # the surface takes part
+
+
+@pytest.mark.parametrize("schedule", ["per_color", "persistent"])
+def test_surface_stiffness_follows_a_captured_refresh(schedule):
+    """A refresh launches kernels only: captured with the step, a replay takes the surface that the model has by then."""
+    model = _block(0.0, False)
+    rng = np.random.default_rng(5)
+    q = model.particle_q + torch.as_tensor(1e-3 * rng.normal(size=(model.particle_count, 3)), device="cuda:0").float()
+    qd = torch.zeros_like(q)
+    solver = SolverVBD(model, iterations=5, schedule=schedule)
+    a, b = model.state(), model.state()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream):
+        a.particle_q.copy_(q)
+        a.particle_qd.copy_(qd)
+        solver.notify_model_changed()
+        solver.step(a, b, None, None, DT)
+    out = []
+    for mu in (0.0, 30.0, 0.0):
+        model.tri_materials[:, :2] = mu
+        graph.replay()
+        torch.cuda.synchronize()
+        out.append(b.particle_q.clone())
+        assert torch.equal(out[-1], _step(SolverVBD(model, iterations=5, schedule=schedule), model, q, qd))
+    assert torch.equal(out[0], out[2]) and not torch.equal(out[0], out[1])
+    del graph
