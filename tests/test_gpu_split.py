@@ -291,3 +291,38 @@ def test_what_steps_split_and_what_does_not():
         assert (SolverVBD(top.finalize("cuda:0"), iterations=4).split is not None) == (worlds < 6 * sms)
     with pytest.raises(KeyError):
         SolverVBD(model, split="on")
+
+
+def test_the_autotuner_times_the_kernels_it_names(monkeypatch):
+    """Every unsplit candidate steps the kernel that it names, the split is a candidate of its own, and what the tuner
+    returns steps as what it timed; a winner that is split carries a launch shape for models too large to split."""
+    from newton_chysx_b200 import autotune
+
+    top = nb.ModelBuilder(up_axis="Z", gravity=-9.81)
+    for n in (9, 12, 16):
+        top.add_world(cloth_grid_builder(n=n))
+    model = top.finalize("cuda:0")
+    built = []
+
+    class Spy(SolverVBD):
+        def __init__(self, *args, **kw):
+            super().__init__(*args, **kw)
+            built.append((kw.get("split"), kw["layout"], self.layout, self.split is not None))
+
+    monkeypatch.setattr(autotune, "SolverVBD", Spy)
+    best = autotune.tune(model, iterations=3, substeps=1)
+    assert sum(is_split for *_, is_split in built) == 1
+    for asked, layout, got, is_split in built:
+        assert layout == got and is_split == (asked != "off")
+    solver = SolverVBD(model, iterations=3, **best)
+    assert (solver.split is None) == (best.get("split") == "off")
+    one = [dict(layout="csr", lanes_per_vertex=2, split="off"), dict(layout="ell16", lanes_per_vertex=1, min_blocks_per_sm=3, split="off"),
+           dict(layout="ell16", lanes_per_vertex=1)]  # fmt: skip
+    for keep, want in ((one, dict(one[1], schedule="persistent")), (one[:2], None)):
+        monkeypatch.setattr(autotune, "candidates", lambda *_: keep)
+        got = autotune.tune(model, iterations=40, substeps=1)
+        if want is not None and "split" not in got:
+            want.pop("split")
+            assert got == want
+        elif want is None:
+            assert got["split"] == "off"
