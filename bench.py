@@ -438,7 +438,8 @@ def run_ours(args):
     if rank == 0 and args.plain_sample > 0:
         plain = run_plain(args, total, shard[: args.plain_sample])
     traffic, traffic_src = args.traffic, "--traffic (ncu capture)" if args.traffic is not None else None
-    if traffic is None and solver.layout in NCU_TRAFFIC_PER_VI:
+    split = solver.split  # batches of fewer than six worlds per SM step in another kernel
+    if traffic is None and split is None and solver.layout in NCU_TRAFFIC_PER_VI:
         per_vi, traffic_src = NCU_TRAFFIC_PER_VI[solver.layout]
         traffic = per_vi * vi_step
     out = None
@@ -472,6 +473,7 @@ def run_ours(args):
                 "block_size": solver.block_size,
                 "positions_in_shared_bytes": solver.shared_bytes,
                 "layout": solver.layout,
+                "split": split,
                 "launch_shape": shape,
                 "autotuned": bool(args.tune),
                 "tune_s": round(tune_s, 1),
@@ -494,7 +496,7 @@ def run_ours(args):
                 "traffic_source": traffic_src,
                 "peak_source": peak_src,
                 "bytes_per_vertex_iteration": bvi,
-                "kernel": "k_persistent (per-substep solve)",
+                "kernel": "k_parts (per-substep solve)" if split else "k_persistent (per-substep solve)",
             },
             "clocks": clocks.summary(),
             "device_errors": errors,
