@@ -245,6 +245,7 @@ struct VbdSolver {
   uint4 *pt_faceA = nullptr, *pt_faceB = nullptr, *pt_hinge = nullptr;
   float *pt_area = nullptr, *pt_length = nullptr, *pt_kd = nullptr;
   int2* pt_place_of = nullptr;
+  unsigned* pt_done = nullptr;
   int* pt_flags = nullptr;
   float4* pt_contact = nullptr;
   // adjoint work buffers (allocated by the first vbd_adjoint_step)
@@ -271,7 +272,7 @@ struct VbdSolver {
                   ell16_faceA, ell16_faceB, ell16_hinge, sc_pos_cd, sc_disp, sc_ts, ring_nslot, ring_base,
                   ring_vbase, ring_A, ring_B, ring_H, ring_hdr, ring_kd, spr_idx, spr_prop, spr_off, spr_adj, sspr_off,
                   sspr_adj, spr_acc, tet_idx, tet_pose, tet_off, tet_adj, sc_estart, sc_world, pt_blob, color_of_dev, live, pt_faceA, pt_faceB, pt_hinge,
-                  pt_area, pt_length, pt_kd, pt_place_of, pt_flags, pt_contact};
+                  pt_area, pt_length, pt_kd, pt_place_of, pt_done, pt_flags, pt_contact};
     for (void* p : ps)
       if (p) cudaFree(p);
     sc_release(sc);
@@ -701,7 +702,7 @@ int upload_plan(VbdSolver* h) {
     blob.insert(blob.end(), b, b + v.size() * sizeof(v[0]));
   };
   PartsView& d = h->pt;
-  put(p.job_order, (const void**)&d.job_order), put(p.part_base, (const void**)&d.part_base);
+  put(p.part_base, (const void**)&d.part_base);
   put(p.vert, (const void**)&d.vert), put(p.start, (const void**)&d.start);
   put(p.ghost_off, (const void**)&d.ghost_off), put(p.ghost, (const void**)&d.ghost);
   put(p.ghost_part, (const void**)&d.ghost_part), put(p.nf, (const void**)&d.nf), put(p.ne, (const void**)&d.ne);
@@ -733,8 +734,7 @@ PartsView parts_view(const VbdSolver* h) {
   p.hinge_kd = h->pt_kd;
   p.flags = h->pt_flags;
   p.contact = h->pt_contact;
-  p.queue = h->queue;
-  p.done = reinterpret_cast<unsigned*>(h->queue + kDoneStride);
+  p.done = h->pt_done;
   return p;
 }
 
@@ -822,13 +822,12 @@ int build_parts(VbdSolver* h, const std::vector<int>& wstart) {
     CK(cudaOccupancyMaxActiveClusters(&fit, fn, &cfg));
   }
   if (fit < 1) return VBD_OK;
-  h->parts.blocks = g.P * (g.grid ? 1 : std::min(fit, h->plan.njobs));
   const size_t nf = size_t(std::max(h->plan.faces, 1LL)), ne = size_t(std::max(h->plan.hinges, 1LL));
   if ((rc = upload_plan(h)) || (h->S > 0 && (rc = dalloc(&h->pt_contact, 3 * size_t(V)))) ||
       (rc = dalloc(&h->pt_place_of, size_t(V))) || (rc = dalloc(&h->pt_faceA, nf)) || (rc = dalloc(&h->pt_faceB, nf)) ||
       (rc = dalloc(&h->pt_area, nf)) || (rc = dalloc(&h->pt_hinge, ne)) || (rc = dalloc(&h->pt_length, ne)) ||
       (rc = dalloc(&h->pt_kd, ne)) ||
-      (rc = dalloc(&h->pt_flags, 1)))
+      (rc = dalloc(&h->pt_flags, 1)) || (g.grid && (rc = dalloc(&h->pt_done, size_t(kDoneStride) * g.P))))
     return rc;
   // places of a round that no element fills stay dead
   CK(cudaMemsetAsync(h->pt_faceA, 0, nf * sizeof(uint4), 0));
@@ -1412,7 +1411,7 @@ int step_impl(VbdSolver* h, R* q_in, R* q_out, const R* qd_in, R* qd_out, const 
     } while (it < iters);
     CK(cudaGetLastError());
   } else if (h->parts_on && !h->sc_on) {
-    CK(cudaMemsetAsync(h->queue, 0, sizeof(int) * (h->parts.grid ? size_t(kDoneStride) * (h->plan.P + 1) : 1), st));
+    if (h->parts.grid) CK(cudaMemsetAsync(h->pt_done, 0, sizeof(unsigned) * size_t(kDoneStride) * h->plan.P, st));
     if (has_c) {
       CK(cudaMemsetAsync(h->slot_cnt, 0, sizeof(int) * h->V, st));
       k_contact_prepare<R><<<(c.c_max + 255) / 256, 256, 0, st>>>(c);
@@ -1981,7 +1980,7 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
                    [&](int a, int b) { return wstart[a + 1] - wstart[a] > wstart[b + 1] - wstart[b]; });
   if ((rc = upload(&h->inst_order, order)) || (rc = upload(&h->inst_vstart, wstart)) ||
       (rc = upload(&h->inst_cptr, cptr)) || (rc = upload(&h->color_ranges, ranges)) ||
-      (rc = upload(&h->color_verts, verts)) || (rc = dalloc(&h->queue, size_t(kDoneStride) * 1025)))
+      (rc = upload(&h->color_verts, verts)) || (rc = dalloc(&h->queue, 1)))
     return fail(rc);
 
   // scratch

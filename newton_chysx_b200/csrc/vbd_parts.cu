@@ -11,7 +11,7 @@
 // the vertices of a color sit next to each other), and L lanes of a warp share a vertex's elements. After a color,
 // vertices that are ghosts elsewhere are written to global memory and fetched from L2 by the parts that read them.
 // Ghosts' first positions need no exchange: every CTA predicts them itself.
-//   grid = false: one job on one cluster, barrier.cluster between colors (up to 1,024 particles: 16 CTAs).
+//   grid = false: the only job on one cluster, barrier.cluster between colors (up to 1,024 particles: 16 CTAs).
 //   grid = true:  the jobs in turn over the whole (cooperative) grid. A part waits only for the parts whose particles
 //                 it reads: each publishes the colors it has finished, and the thread that fetches a ghost polls its
 //                 owner's flag (bounded). Two parts that share an element read each other's particles, in two colors
@@ -361,7 +361,6 @@ __global__ void __launch_bounds__(T, 1)
     k_parts(const __grid_constant__ StepCtx<R> c, const __grid_constant__ PartsView p, int grid_mode, int iterations) {
   extern __shared__ __align__(32) unsigned char s_raw[];
   pos4_t<R>* s_pos = reinterpret_cast<pos4_t<R>*>(s_raw);
-  __shared__ int s_item;
   __shared__ PartShared s;
   namespace cg = cooperative_groups;
   const int rank = grid_mode ? int(blockIdx.x) : int(cg::this_cluster().block_rank());
@@ -369,22 +368,8 @@ __global__ void __launch_bounds__(T, 1)
   const int flags = *p.flags;
   unsigned phase = 0;
   if (tid == 0) s.abort = 0;
-  for (int round = 0;; ++round) {
-    int job = 0;
-    if (grid_mode) {
-      if (round >= p.njobs) return;
-      job = round;
-      __syncthreads();
-    } else {
-      cluster_barrier();
-      if (rank == 0 && tid == 0) {
-        const int q = atomicAdd(p.queue, 1);
-        for (int b = 0; b < p.P; ++b) *cg::this_cluster().map_shared_rank(&s_item, b) = q;
-      }
-      cluster_barrier();
-      if (s_item >= p.njobs) return;
-      job = __ldg(p.job_order + s_item);
-    }
+  for (int job = 0; job < p.njobs; ++job) {
+    __syncthreads();
     const int part = job * p.P + rank;
     const int v0 = __ldg(p.part_base + part), nown = __ldg(p.part_base + part + 1) - v0;
     const int* go = p.ghost_off + size_t(part) * (p.C + 1);
@@ -472,7 +457,7 @@ template <typename R, int MODE>
 cudaError_t launch_parts(const PartsConfig& g, const StepCtx<R>& c, const PartsView& p, int iterations, cudaStream_t st) {
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(g.blocks);
+  cfg.gridDim = dim3(g.P);
   cfg.blockDim = dim3(g.block);
   cfg.dynamicSmemBytes = g.smem;
   cfg.stream = st;

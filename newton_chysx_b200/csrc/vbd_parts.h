@@ -16,7 +16,6 @@ struct PartsView {
   int njobs;
   const int* flags;           // kFaceDamping, kHingeDamping, kFloor (a refresh rewrites it)
   int places, most_own;       // most places and most own particles of a part: the shared-memory layout
-  const int* job_order;       // [njobs] largest first
   const int* part_base;       // [parts + 1] own particles of all parts before
   const int* vert;            // [V] particle of part-local place s at part_base + s; bit 31: ghost of another part
   const int* start;           // [parts, C + 1] own places by color
@@ -36,7 +35,6 @@ struct PartsView {
   const float* hinge_length;  // read in FP64
   const float* hinge_kd;      // read with kHingeDamping or kFloor
   float4* contact;            // [3 V] by place: a particle's only contact with a static shape, as part_contact_add reads it
-  int* queue;                 // work counter, zero before launch
   unsigned* done;             // [P * kDoneStride] colors finished by each CTA over its jobs, zero before launch (grid)
 };
 
@@ -55,11 +53,10 @@ constexpr int kPartColors = 32;  // most colors of a plan
 
 struct PartsConfig {
   int P = 0;           // parts per job
-  bool grid = false;   // jobs in turn over the whole grid (cooperative launch); else a job per cluster
+  bool grid = false;   // jobs in turn over the whole grid (cooperative launch); else one job on one cluster
   int L = 1;           // lanes per vertex
   bool wide = false;   // the variant for up to 896 threads (72 registers) instead of 512 (128 registers)
   int block = 0;
-  int blocks = 0;      // CTAs of the launch
   size_t smem = 0;
 };
 
@@ -82,7 +79,7 @@ struct PartsInput {
 };
 struct PartsPlan {
   int P = 0, L = 1, njobs = 0, C = 0, most_places = 0, most_own = 0;
-  std::vector<int> job_order, part_base, part_of, slot_of, vert, start, ghost_off, ghost, ghost_part, nf, ne;
+  std::vector<int> part_base, part_of, slot_of, vert, start, ghost_off, ghost, ghost_part, nf, ne;
   std::vector<long long> fbase, ebase;
   long long faces = 0, hinges = 0;
 };

@@ -63,11 +63,6 @@ bool parts_plan(const PartsInput& in, const std::vector<int>& job_v0, int P, int
   plan.P = P, plan.L = L, plan.C = C;
   plan.njobs = int(job_v0.size()) - 1;
   const int parts = plan.njobs * P;
-  plan.job_order.resize(plan.njobs);
-  for (int j = 0; j < plan.njobs; ++j) plan.job_order[j] = j;
-  std::stable_sort(plan.job_order.begin(), plan.job_order.end(), [&](int a, int b) {
-    return job_v0[a + 1] - job_v0[a] > job_v0[b + 1] - job_v0[b];
-  });
   plan.part_of.assign(V, 0);
   plan.slot_of.assign(V, 0);
   plan.vert.assign(V, 0);
