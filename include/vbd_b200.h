@@ -191,7 +191,9 @@ int vbd_step_f64(VbdHandle h, double* q_in_dev, double* q_out_dev, const double*
    the end. Arrays are float32, or float64 for a VBD_PRECISION_FP64 solver. q_out/qd_out receive the step's
    result (q_in is not modified). contacts: this substep's particle-shape contacts against static shapes, or
    NULL; the adjoint must be given the same arrays. Membranes, hinges, tetrahedra and springs with their damping
-   take part. VBD_ERR_UNSUPPORTED for contacts with the AVBD penalty ramp on (rigid_avbd_beta > 0). */
+   take part. VBD_ERR_UNSUPPORTED for contacts with the AVBD penalty ramp on (rigid_avbd_beta > 0);
+   VBD_ERR_INVALID_ARGUMENT when the colors do not list every particle once (a checkpoint pair then does not hold
+   the states between the colors). */
 int vbd_record_step(VbdHandle h, const void* q_in_dev, const void* qd_in_dev, const void* particle_f_dev,
                     const VbdContactsDesc* contacts, double dt, void* y_dev, void* checkpoints_dev, void* q_out_dev,
                     void* qd_out_dev, void* stream);
@@ -200,8 +202,8 @@ int vbd_record_step(VbdHandle h, const void* q_in_dev, const void* qd_in_dev, co
    and dL/dqd_in and ADDS the triangles' dL/dmu and dL/dlambda (Model.tri_materials columns 0 and 1)
    into adj_tri_mu / adj_tri_lambda [T] (either may be NULL). contacts: the arrays the forward substep was
    given; their contact set, points, normals and stiffness are held fixed (the derivative of the step for
-   those contacts). The first call allocates (colors + 3) x V x 3 work values; it returns
-   VBD_ERR_UNSUPPORTED if that happens during a capture. */
+   those contacts). The first call allocates 3 x V x 3 work values; it returns VBD_ERR_UNSUPPORTED if that
+   happens during a capture. */
 int vbd_adjoint_step(VbdHandle h, const void* q_in_dev, const void* y_dev, const void* checkpoints_dev,
                      const VbdContactsDesc* contacts, double dt, const void* adj_q_out_dev,
                      const void* adj_qd_out_dev, void* adj_q_in_dev, void* adj_qd_in_dev, void* adj_tri_mu_dev,

@@ -239,6 +239,7 @@ struct VbdSolver {
   PartsConfig parts;
   PartsPlan plan;
   std::vector<int> color_of;  // [V] place of each particle's color in the sweep
+  bool one_color_each = true;  // every particle is listed once by the colors
   int* color_of_dev = nullptr;
   PartsView pt = {};
   char* pt_blob = nullptr;
@@ -1907,9 +1908,12 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
   if ((rc = dalloc(&h->tri_idx, h->T)) || (rc = dalloc(&h->tri_pose, h->T)) || (rc = dalloc(&h->tri_mat, h->T)) ||
       (rc = dalloc(&h->edge_idx, h->E)) || (rc = dalloc(&h->edge_prop, h->E)))
     return fail(rc);
-  h->color_of.assign(h->V, 0);
+  // -1: a particle that no color lists (another one is listed twice) is never solved; the split and the recorded substep
+  // need every particle in one color
+  h->color_of.assign(h->V, -1);
   for (size_t col = 0; col + 1 < h->color_offsets.size(); ++col)
     for (int k = h->color_offsets[col]; k < h->color_offsets[col + 1]; ++k) h->color_of[colp[k]] = int(col);
+  h->one_color_each = std::find(h->color_of.begin(), h->color_of.end(), -1) == h->color_of.end();
   if ((rc = upload(&h->color_of_dev, h->color_of))) return fail(rc);
   if (soft) {
     const std::vector<int>& color_of = h->color_of;
@@ -1918,7 +1922,7 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
                          ssadj);
     h->n_same_springs = ssoff[h->V];
     for (int v = 0; v < h->V; ++v)
-      if (ssoff[v + 1] > ssoff[v]) h->same_colors |= 1ull << std::min(color_of[v], 63);
+      if (ssoff[v + 1] > ssoff[v] && color_of[v] >= 0) h->same_colors |= 1ull << std::min(color_of[v], 63);
     if ((rc = dalloc(&h->live, 2))) return fail(rc);
     const size_t racc = h->precision == VBD_PRECISION_FP64 ? sizeof(double) : sizeof(float);
     if ((rc = upload(&h->tet_off, toff)) || (rc = upload(&h->tet_adj, tadj)) || (rc = upload(&h->spr_off, soff)) ||
@@ -2079,7 +2083,7 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
   // positions off or on) keep it
   const bool plain = params->layout == VBD_LAYOUT_AUTO && lpv == 0 && params->block_size == 0 &&
                      params->min_blocks_per_sm == 0 && params->positions_in_shared == 0;
-  if (!soft && !lnh_floor && params->split == 0 && params->schedule != VBD_SCHEDULE_PER_COLOR && params->pair_vertices == 0 &&
+  if (!soft && !lnh_floor && h->one_color_each && params->split == 0 && params->schedule != VBD_SCHEDULE_PER_COLOR && params->pair_vertices == 0 &&
       params->instance_per_warp == 0 && (plain || h->layout == VBD_LAYOUT_ELL16)) {
     if ((rc = build_parts(h, wstart))) return fail(rc);
   }
@@ -2187,6 +2191,7 @@ int vbd_record_step(VbdHandle h, const void* q_in, const void* qd_in, const void
                     const VbdContactsDesc* contacts, double dt, void* y, void* checkpoints, void* q_out, void* qd_out,
                     void* stream) {
   if (!h || !q_in || !qd_in || !y || !checkpoints || !q_out || !qd_out || !(dt > 0.0)) return VBD_ERR_INVALID_ARGUMENT;
+  if (!h->one_color_each) return VBD_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   if (h->precision == VBD_PRECISION_FP64)
     return record_impl<double>(h, (const double*)q_in, (const double*)qd_in, (const double*)particle_f, contacts, dt,
@@ -2199,6 +2204,7 @@ int vbd_adjoint_step(VbdHandle h, const void* q_in, const void* y, const void* c
                      const VbdContactsDesc* contacts, double dt, const void* adj_q_out, const void* adj_qd_out,
                      void* adj_q_in, void* adj_qd_in, void* adj_tri_mu, void* adj_tri_lambda, void* stream) {
   if (!h || !q_in || !y || !checkpoints || !adj_q_in || !(dt > 0.0)) return VBD_ERR_INVALID_ARGUMENT;
+  if (!h->one_color_each) return VBD_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   if (h->precision == VBD_PRECISION_FP64)
     return adjoint_impl<double>(h, (const double*)q_in, (const double*)y, (const double*)checkpoints, contacts, dt,

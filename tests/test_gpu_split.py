@@ -249,6 +249,28 @@ def test_split_refresh_takes_materials_under_the_floor(precision):
     assert (got - ref).abs().max().item() <= (1e-9 if precision == "fp64" else 1e-5)
 
 
+def test_a_particle_without_a_color_is_not_solved():
+    """Colors that list one particle twice and another never: the latter takes its inertial target, on every schedule, and
+    the recorded substep, whose checkpoints could not hold the states between the colors, refuses the model."""
+    from newton_chysx_b200.adjoint import DifferentiableVBD
+
+    b = cloth_grid_builder(n=12, hanging=False, height=1.0)
+    groups = [np.sort(np.int32(g)) for g in b.particle_color_groups]
+    left_out, groups[1] = int(groups[1][3]), np.concatenate([groups[1][:3], groups[1][4:], groups[0][5:6]])
+    b.set_coloring(groups)
+    model = b.finalize("cuda:0")
+    q, qd = _start(model, 1)
+    target = q[left_out] + DT * (qd[left_out] + DT * np.float32([0.0, 0.0, -9.81]))
+    for kw in ({}, dict(schedule="per_color", layout="csr"), dict(schedule="persistent", layout="ell")):
+        assert SolverVBD(model, **kw).split is None
+        got, _ = _run(model, q, qd, substeps=1, **kw)
+        assert np.abs(got[left_out] - target).max() <= 1e-6  # FP32 positions of up to 1.1 m
+    sim = DifferentiableVBD(model, iterations=3)
+    mu, lam = model.tri_materials[:, 0].clone(), model.tri_materials[:, 1].clone()
+    with pytest.raises(_lib.VbdError, match="invalid argument"):
+        sim.rollout(torch.as_tensor(q, device="cuda"), torch.as_tensor(qd, device="cuda"), mu, lam, DT, 1)
+
+
 def test_what_steps_split_and_what_does_not():
     """The split is reported, taken with the default options and with ell16 whatever its launch shape, and left where an
     option names another kernel, split="off" asks for it, there is nothing to split or enough worlds fill the GPU."""
