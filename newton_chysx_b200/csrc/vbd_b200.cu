@@ -780,15 +780,24 @@ int build_parts(VbdSolver* h, const std::vector<int>& wstart) {
   for (int w = 1; w < W; ++w)
     if ((long long)wstart[w] * nj >= (long long)V * (long long)job_v0.size()) job_v0.push_back(wstart[w]);
   job_v0.push_back(V);
-  int per_color = 1;  // the longest run of a color in a part
+  int per_color = 1;         // the longest run of a color in a part
+  long long most_own = 0;  // the most particles of a part
   {
     std::vector<int> count(C);
     for (size_t j = 0; j + 1 < job_v0.size(); ++j) {
       std::fill(count.begin(), count.end(), 0);
       for (int v = job_v0[j]; v < job_v0[j + 1]; ++v) ++count[h->color_of[v]];
-      for (int c = 0; c < C; ++c) per_color = std::max(per_color, (count[c] + g.P - 1) / g.P);
+      long long own = 0;
+      for (int c = 0; c < C; ++c) {
+        per_color = std::max(per_color, (count[c] + g.P - 1) / g.P);
+        own += (count[c] + g.P - 1) / g.P;
+      }
+      most_own = std::max(most_own, own);
     }
   }
+  // no plan for parts that do not fit without their ghosts (sheets from about 0.9 M particles on in FP32): it takes the
+  // host a second
+  if (size_t(std::max(0LL, most_own - C)) * (2 * place + sizeof(int)) + 2048 > size_t(optin)) return VBD_OK;
   // as many lanes per vertex as leave one round of a run (256 x 256: 421 us with 4, 511 with 8 in two rounds, 469
   // with 2); two lanes also where that takes the wide variant (512 x 512 mixed: 1.77 ms against 2.01 with 1)
   g.L = 1;
@@ -2086,6 +2095,7 @@ int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHand
   if (!soft && !lnh_floor && h->one_color_each && params->split == 0 && params->schedule != VBD_SCHEDULE_PER_COLOR && params->pair_vertices == 0 &&
       params->instance_per_warp == 0 && (plain || h->layout == VBD_LAYOUT_ELL16)) {
     if ((rc = build_parts(h, wstart))) return fail(rc);
+    if (!h->parts_on) h->plan = PartsPlan();
   }
   if (!h->parts_on &&
       (h->layout == VBD_LAYOUT_ELL || h->layout == VBD_LAYOUT_ELL16 || h->layout == VBD_LAYOUT_RING)) {
