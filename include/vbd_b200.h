@@ -165,7 +165,9 @@ typedef struct VbdSolver* VbdHandle;
 int vbd_create(const VbdModelDesc* model, const VbdSolverParams* params, VbdHandle* out);
 
 /* Re-reads the model arrays given to vbd_create (materials, rest state, masses, flags) after the
-   caller changed them in place; replaces SolverVBD.notify_model_changed (solver_vbd.py:779-782). */
+   caller changed them in place; replaces SolverVBD.notify_model_changed (solver_vbd.py:779-782). On the CSR layout,
+   split or not, it launches kernels on `stream` only and may be captured; the stencil layouts check the materials
+   (VBD_ERR_UNSUPPORTED) or rebuild their records on the host and synchronise `stream`. */
 int vbd_refresh_model(VbdHandle h, void* stream);
 
 /* Replaces SolverVBD.step(state_in, state_out, control, contacts, dt) for particles

@@ -20,15 +20,16 @@
 //                 atomic counter) cost about 3 us per color.
 //
 // Measured, us per substep (collide + step), before and after, 10 iterations unless said:
-//   32 x 32 FP32          1,557 -> 149   (one CTA, 8 lanes per vertex, before)
+//   32 x 32 FP32          1,557 -> 145   (one CTA, 8 lanes per vertex, before)
 //   161 x 97 FP32           517 -> 173   (40 launches of one lane per vertex)
-//   256 x 256 FP32, 20 it 1,025 -> 421
-//   512 x 512 mixed, 30 it 2,605 -> 1,768
-//   96 x 96 FP64            791 -> 229
-//   60 worlds of 16..40 squared, damped 1,126 -> 333 (one CTA per world before)
-//   512 worlds of 16..128 squared (3.3 M particles) 10,101 -> 5,345: seven jobs; issue and the records' stream from
+//   256 x 256 FP32, 20 it 1,025 -> 426
+//   512 x 512 mixed, 30 it 2,605 -> 1,772
+//   96 x 96 FP64            791 -> 251
+//   60 worlds of 16..40 squared, damped 1,126 -> 342 (one CTA per world before)
+//   512 worlds of 16..128 squared (3.3 M particles) 10,101 -> 5,296: seven jobs; issue and the records' stream from
 //   HBM bound it, 6.2e9 vertex-iterations/s
-// What bounds the small ones now is the serial chain of a color: about 4 us of dependent instructions and loads.
+// What bounds the small ones now is the serial chain of a color: about 4 us of dependent instructions and loads (161 x 97:
+// 19 % of issue slots used, 2.7 barrier and 2.0 long-scoreboard stalls per issue).
 #include "vbd_parts.h"
 
 #include <cooperative_groups.h>

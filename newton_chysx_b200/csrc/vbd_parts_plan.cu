@@ -151,8 +151,9 @@ __global__ void k_parts_places(const PartsView p, int2* place_of) {
   for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) place_of[p.vert[k] & 0x7fffffff] = make_int2(part, k - k0);
 }
 
-// A block per part and slice of its particles, a thread per particle. A refresh of 512 worlds of side U{16..128} (3.3 M
-// particles, 1.3 GB of records) replaces 1.1 s of host loops and uploads.
+// A block per part and slice of its particles, a thread per particle. Bound by the scattered reads of elements and places;
+// a refresh of a 256 x 256 sheet takes 1.1 ms with it (12 ms with the records built on the host and uploaded), of 512
+// worlds of side U{16..128} (3.3 M particles, 1.3 GB of records) 83 ms, most of it the check of the materials (901 ms).
 constexpr int kPackSlices = 4;
 template <bool F64>
 __global__ void __launch_bounds__(256) k_parts_pack(const PartsModel m, const PartsView p, int L, const PartsRecords r) {
