@@ -120,6 +120,26 @@ def test_split_fp64_holds_elements_as_the_csr_kernel_does(nx, ny, kd):
     assert np.abs(got - ref).max() <= 2e-15 and np.abs(got_d - ref_d).max() <= 2e-15 / DT
 
 
+@pytest.mark.parametrize("shared", ["on", "off"])
+@pytest.mark.parametrize("kd", [0.0, 1e-3])
+@pytest.mark.parametrize("precision", ["fp32", "mixed"])
+def test_unsplit_ell16_worlds_match_fp64(precision, kd, shared):
+    """The kernel of large batches, one CTA per world on 16-bit records, with and without hinge damping (two kernels) and
+    positions in shared memory: FP32 sums against FP64 over one substep, 1e-4 m per m as every FP32 kernel here."""
+    top = nb.ModelBuilder(up_axis="Z", gravity=-9.81)
+    for n in (17, 30, 9, 64):
+        top.add_world(_sheet(n, n, kd, shapes=0))
+    top.add_ground_plane(cfg=nb.ModelBuilder.ShapeConfig(ke=1e4, kd=1e-4, mu=0.5))
+    model = top.finalize("cuda:0")
+    model.soft_contact_ke, model.soft_contact_kd, model.soft_contact_mu = 1e4, 1e-4, 0.5
+    q, qd = _start(model, 4)
+    kw = dict(schedule="persistent", layout="ell16", split="off")
+    assert SolverVBD(model, precision=precision, positions_in_shared=shared, **kw).split is None
+    got, _ = _run(model, q, qd, substeps=1, precision=precision, positions_in_shared=shared, **kw)
+    ref, _ = _run(model, q, qd, substeps=1, precision="fp64", schedule="persistent", layout="csr")
+    assert np.abs(got - ref).max() <= 1e-4
+
+
 def _damp(model, faces, hinges):
     model.tri_materials[:, 2] = faces
     model.edge_bending_properties[:, 1] = hinges
